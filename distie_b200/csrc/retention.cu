@@ -23,7 +23,6 @@
 
 namespace distie {
 
-constexpr int kChunk = 64;
 constexpr int kReadThreads = 512;    // 16 warps: four groups of 16 rows by four groups of columns
 constexpr int kWriteThreads = 256;   // (three blocks an SM)
 
@@ -46,22 +45,6 @@ __device__ __forceinline__ float power_of(float x, int n) {  // x^n, n >= 0
     x *= x;
   }
   return out;
-}
-
-// D[16 x 8] += A[16 x 16] B[16 x 8]; with g = lane / 4, c = lane % 4: d = D[g][2c], D[g][2c+1], D[g+8][2c], D[g+8][2c+1].
-__device__ __forceinline__ void mma_16bit(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void load_matrices(uint32_t (&r)[4], const __nv_bfloat16* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
-}
-__device__ __forceinline__ void load_matrices_turned(uint32_t (&r)[4], const __nv_bfloat16* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
 
 // A matrix in shared memory as two bfloat16 parts, `ld` elements a row; rows start an odd number of 16-byte pieces apart,
@@ -90,7 +73,6 @@ struct Parts {
         make_uint2(*reinterpret_cast<const uint32_t*>(&l0), *reinterpret_cast<const uint32_t*>(&l1));
   }
 };
-__host__ __device__ constexpr int up16(int n) { return (n + 15) & ~15; }
 __host__ __device__ constexpr int parts_ld(int columns) { return up16(columns) + 8; }
 __host__ __device__ constexpr size_t parts_bytes(int rows, int columns) { return (size_t)2 * rows * parts_ld(columns) * 2; }
 __device__ __forceinline__ Parts parts_at(unsigned char*& at, int rows, int columns) {
@@ -202,13 +184,6 @@ __device__ __forceinline__ void load_values(const RetentionArgs& a, int t0, int 
       dst.put(r, e, weight_s ? x * weight_s[r] : x);
     }
   }
-}
-
-// Where chunk `chunk` of the step lies: its first token and its number of tokens (0: the second half of a short tile).
-__device__ __forceinline__ int chunk_rows(const int* q_tiles, int chunk, int& t0) {
-  const int tile = chunk >> 1, half = chunk & 1;
-  t0 = q_tiles[2 * tile] + half * kChunk;
-  return min(kChunk, q_tiles[2 * tile + 1] - half * kChunk);
 }
 
 // U^T [value_dim, key_dim] of a chunk: rows are value elements (V^T is the first operand), columns key elements.

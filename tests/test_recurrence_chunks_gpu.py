@@ -1,0 +1,101 @@
+"""Linear recurrences of long portions (chunks on the tensor cores) against the token-by-token formulas in 64 bits.
+
+The operands enter in three bfloat16 parts, which hold the 24 bits of a float32, so what is left is the rounding of
+float32 sums and of a chunk's products of decays: at most 64 factors and 128 terms of 2^-24 each, in quadrature about
+14 * 2^-24 = 8e-7 of the result; the bound is twice that.  The walk is held to the same bound."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from test_kernels_gpu import step_of
+
+pytestmark = pytest.mark.gpu
+
+BOUND = 1.7e-6
+
+
+def exact(rule, p, lengths, order, heads, groups, key_dim, value_dim, unit):
+    double = {n: t.double() if t is not None else None for n, t in p.items()}
+    wide = lambda x: x.reshape(-1, groups, key_dim).repeat_interleave(heads // groups, 1)  # noqa: E731
+    q, k = wide(double["q"]), wide(double["k"])
+    v = double["v"].reshape(q.shape[0], heads, -1)
+    if unit:
+        v = torch.cat([v, torch.ones_like(v[..., :1])], -1)
+    softplus = torch.nn.functional.softplus
+    if rule == "gated":
+        g = double["decay"] if double["decay"] is not None else double["rate"].expand(q.shape[0], -1)
+        factor = double["write"] if double["write"] is not None else torch.ones_like(g)
+    elif rule == "ssd":
+        factor = softplus(double["write"] + double["bias"])
+        g = torch.exp(-double["rate"].exp() * factor)
+    else:
+        factor = torch.sigmoid(double["write"])
+        g = torch.exp(-double["rate"].exp() * softplus(double["decay"] + double["bias"]))
+        q = q / (q.square().sum(-1, keepdim=True) + 1e-6).sqrt() * key_dim**-0.5
+        k = k / (k.square().sum(-1, keepdim=True) + 1e-6).sqrt()
+    out = torch.empty(q.shape[0], heads, value_dim, dtype=torch.float64, device="cuda")
+    states, start = double["state"].clone(), 0
+    for row in order:
+        S = states[row]
+        for t in range(start, start + lengths[row]):
+            S = S * g[t, :, None, None]
+            held = torch.einsum("hvk,hk->hv", S, k[t]) if rule == "delta" else 0.0
+            S = S + (factor[t, :, None] * (v[t] - held))[:, :, None] * k[t][:, None]
+            out[t] = torch.einsum("hvk,hk->hv", S, q[t])
+            if rule == "ssd":
+                out[t] += double["skip"][:, None] * v[t]
+        states[row] = S
+        start += lengths[row]
+    return out.reshape(q.shape[0], -1), states
+
+
+# lengths, heads, groups, key size, value size: whole and ragged chunks, a token alone beside portions, sizes that fill no
+# tile and no vector, the largest sizes taken, and one key size beyond them (the walk)
+SIZES = [
+    ([490], 4, 4, 128, 128),
+    ([1, 257, 1, 193, 320], 4, 2, 64, 96),
+    ([917], 2, 1, 50, 33),
+    ([961], 2, 2, 17, 144),
+    ([513, 64, 700], 3, 3, 128, 129),
+    ([300], 2, 2, 160, 64),
+]
+
+
+@pytest.mark.parametrize("lengths,heads,groups,key_dim,value_dim", SIZES)
+@pytest.mark.parametrize("rule,strong", [("ssd", False), ("ssd", True), ("gated", False), ("gated", True), ("constant", False)])
+def test_chunks_of_a_recurrence(rule, strong, lengths, heads, groups, key_dim, value_dim):
+    from distie_b200.kernels import make_kernels
+
+    ks = make_kernels(torch.bfloat16, "cuda:0")
+    generator = torch.Generator(device="cuda").manual_seed(7)
+    normal = lambda *shape: torch.randn(*shape, generator=generator, device="cuda")  # noqa: E731
+    total, constant = sum(lengths), rule == "constant"
+    rule = "gated" if constant else rule
+    unit = rule == "gated" and value_dim == 129
+    p = {"q": normal(total, groups * key_dim), "k": normal(total, groups * key_dim) + 0.3,
+         "v": normal(total, heads * (value_dim - unit)), "decay": normal(total, heads), "write": normal(total, heads),
+         "rate": normal(heads) * 0.5, "bias": normal(heads) - 3, "skip": None,
+         "state": normal(len(lengths), heads, value_dim, key_dim)}
+    if rule == "ssd":
+        p["skip"] = normal(heads)
+        p["bias"] += 6 if strong else 0  # strong: a token forgets nearly all that was before it
+    elif rule == "gated" and not constant:
+        p["decay"], p["write"] = torch.exp(-p["decay"] ** 2 * (9 if strong else 0.02)), torch.sigmoid(p["write"])
+        if strong:
+            p["decay"][normal(total, heads) > 2] = 0.0
+    if constant:
+        p["decay"] = p["write"] = None
+        p["rate"] = torch.linspace(0.75, 0.996, heads, device="cuda")
+    step = step_of(lengths, [3] * len(lengths), list(range(len(lengths))))
+    order = sorted(range(len(lengths)), key=lambda i: (lengths[i] != 1, i))
+    want, want_state = exact(rule, p, lengths, order, heads, groups, key_dim, value_dim, unit)
+    state = p["state"].clone()
+    got = ks.linear_recurrence(rule, p["q"].clone(), p["k"].clone(), p["v"], p["decay"], p["write"], state, step, heads, groups,
+                               key_dim, value_dim, decay_rate=p["rate"], decay_bias=p["bias"] if rule != "gated" else None,
+                               skip=p["skip"], unit_column=unit)
+    assert ("recurrence_chunks" in ks.kernel_counts) == (key_dim <= 128)
+    for name, a, b in (("read-out", got, want), ("state", state, want_state)):
+        error = float((a.double() - b).norm() / b.norm())
+        assert error <= BOUND, f"{rule} {name}: off by {error:.2e}"

@@ -33,7 +33,6 @@ _CLUSTER_SPLITS = 8             # splits of a decode attention that one cluster 
 _TENSOR_CORE_ROWS = 128         # from here on the tcgen05 kernel's 128-row tiles are full; in between: the library
 _MAX_TERMS = 24                 # terms of a pending sum that the layer-norm kernel adds up itself
 _RULES = {"delta": 0, "ssd": 1, "gated": 2}
-_CHUNK_RULES = ("ssd", "gated")
 _CHUNK_BYTES = 1 << 30          # the most that the states between the chunks of a step may take
 _ACTS = {"relu2": 1, "gelu": 2, "xielu": 3}
 _SCORINGS = {"sigmoid": 0, "softmax": 1, "softmax_chosen": 2}
@@ -681,9 +680,10 @@ class DeviceKernels(KernelSet):
         96 38 / 35; sixteen of 33 54 / 65, of 64 92 / 70.  The line below lies between these."""
         singles = step.num_decode_tokens
         portions, rest = step.num_seqs - singles, step.num_tokens - singles
-        return (rule in _CHUNK_RULES and self.dtype == torch.bfloat16 and portions > 0 and step.num_q_tiles > 0
+        return (self.dtype == torch.bfloat16 and portions > 0 and step.num_q_tiles > 0
                 and rest >= 48 * portions + 1700 / heads and key_dim <= 128 and value_dim <= 144 and state.is_contiguous()
-                and 8 * step.num_q_tiles * heads * key_dim * value_dim <= _CHUNK_BYTES)
+                and 4 * function("distie_recurrence_chunks_scratch_floats")(_RULES[rule], step.num_q_tiles, heads, key_dim,
+                                                                            value_dim) <= _CHUNK_BYTES)
 
     def gated_rmsnorm(self, x, gate, weight, eps, group, gate_first, out, activation="silu") -> None:
         self._rows32(x, "gated_rmsnorm x")

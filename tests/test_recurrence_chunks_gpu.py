@@ -64,7 +64,8 @@ SIZES = [
 
 
 @pytest.mark.parametrize("lengths,heads,groups,key_dim,value_dim", SIZES)
-@pytest.mark.parametrize("rule,strong", [("ssd", False), ("ssd", True), ("gated", False), ("gated", True), ("constant", False)])
+@pytest.mark.parametrize("rule,strong", [("delta", False), ("delta", True), ("ssd", False), ("ssd", True),
+                                         ("gated", False), ("gated", True), ("constant", False)])
 def test_chunks_of_a_recurrence(rule, strong, lengths, heads, groups, key_dim, value_dim):
     from distie_b200.kernels import make_kernels
 
@@ -78,6 +79,8 @@ def test_chunks_of_a_recurrence(rule, strong, lengths, heads, groups, key_dim, v
          "v": normal(total, heads * (value_dim - unit)), "decay": normal(total, heads), "write": normal(total, heads),
          "rate": normal(heads) * 0.5, "bias": normal(heads) - 3, "skip": None,
          "state": normal(len(lengths), heads, value_dim, key_dim)}
+    if rule == "delta" and strong:  # hardly anything is forgotten and all is corrected: the longest way through a chunk
+        p["bias"], p["write"] = p["bias"] - 3, p["write"].abs() + 3
     if rule == "ssd":
         p["skip"] = normal(heads)
         p["bias"] += 6 if strong else 0  # strong: a token forgets nearly all that was before it

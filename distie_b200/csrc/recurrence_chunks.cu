@@ -27,11 +27,13 @@
 // Why chunks: the walk is a chain of about 110 dependent instructions a token and head column, 0.15 to 0.25 us a token
 // whatever the machine could do beside it.  Single tokens and short portions stay on it (the rule is in kernels/device.py).
 #include "recurrent.cuh"
+#include "tcgen05.cuh"
 
 namespace distie {
 
-constexpr int kWideThreads = 512;   // read: one block an SM, 16 warps
-constexpr int kNarrowThreads = 256; // write: two blocks an SM
+constexpr int kChunkThreads = 256;  // write, solve: two blocks an SM
+constexpr int kWideThreads = 512;   // read: one
+constexpr int kChunkWarps = kChunkThreads / 32;
 constexpr int kKeyPitch = 128;      // elements a row of a matrix over the key's elements
 constexpr int kBlocks = kChunk / 16;
 constexpr int kImage = 3 * kChunk * kKeyPitch;  // elements of one image
@@ -50,6 +52,7 @@ struct ChunkArgs {
   int out_stride;
   const int *q_tiles, *token_seq, *seq_seat;
   int tiles, heads, groups, key_dim, value_dim, v_dim;
+  int* error;
 };
 
 constexpr int kRuleDelta = 0, kRuleSsd = 1, kRuleGated = 2;
@@ -66,19 +69,26 @@ __device__ __forceinline__ void three_parts(float x, float y, uint32_t (&out)[3]
 }
 
 // A matrix as three bfloat16 parts, in shared memory or as an image of it.  Pieces of eight columns are swapped by the
-// row's last three bits, so that the eight rows of an ldmatrix lie in different banks; a row is a multiple of 64 elements.
+// row's last three bits, so that the eight rows of an ldmatrix lie in different banks.  PITCH: elements of a row, a multiple
+// of 64; ROWS: of a part, in elements PITCH * ROWS.  A step of 16 columns is a flip of address bits (stepped) where the
+// columns start at 0 and the pitch is a power of two.
+template <int PITCH, int ROWS>
 struct Triple {
   __nv_bfloat16* p;
-  int pitch, part;  // elements of a row, of a part
-  __device__ __forceinline__ int at(int row, int col) const { return row * pitch + ((((col >> 3) ^ (row & 7)) << 3) | (col & 7)); }
+  static constexpr int kPitch = PITCH, kPart = PITCH * ROWS;
+  static constexpr size_t kBytes = 3 * (size_t)kPart * 2;
+  static __device__ __forceinline__ int at(int row, int col) { return row * PITCH + ((((col >> 3) ^ (row & 7)) << 3) | (col & 7)); }
 };
 // The same with 16 columns: rows lie 48 bytes apart, which keeps an ldmatrix's rows in different banks by itself.
+template <int ROWS>
 struct NarrowTriple {
   __nv_bfloat16* p;
-  int part;
-  static constexpr int kPitch = 24;
-  __device__ __forceinline__ int at(int row, int col) const { return row * kPitch + col; }
+  static constexpr int kPitch = 24, kPart = kPitch * ROWS;
+  static constexpr size_t kBytes = 3 * (size_t)kPart * 2;
+  static __device__ __forceinline__ int at(int row, int col) { return row * kPitch + col; }
 };
+using KeyTriple = Triple<kKeyPitch, kChunk>;  // 64 tokens by the key's elements
+using SquareTriple = Triple<kChunk, kChunk>;
 template <class M>
 __device__ __forceinline__ void put4(const M& m, int row, int col, float4 x) {  // col a multiple of 4
   uint32_t a[3], b[3];
@@ -86,7 +96,7 @@ __device__ __forceinline__ void put4(const M& m, int row, int col, float4 x) {  
   three_parts(x.z, x.w, b);
   __nv_bfloat16* to = m.p + m.at(row, col);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(to + i * m.part) = make_uint2(a[i], b[i]);
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(to + i * M::kPart) = make_uint2(a[i], b[i]);
 }
 template <class M>
 __device__ __forceinline__ void put2(const M& m, int row, int col, float x, float y) {  // col even
@@ -94,43 +104,43 @@ __device__ __forceinline__ void put2(const M& m, int row, int col, float x, floa
   three_parts(x, y, a);
   __nv_bfloat16* to = m.p + m.at(row, col);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(to + i * m.part) = a[i];
-}
-__host__ __device__ constexpr int value_pitch(int value_dim) { return (value_dim + 63) / 64 * 64; }
-__host__ __device__ constexpr size_t triple_bytes(int rows, int pitch) { return (size_t)3 * rows * pitch * 2; }
-__device__ __forceinline__ Triple triple_at(unsigned char*& at, int rows, int pitch) {
-  Triple t{reinterpret_cast<__nv_bfloat16*>(at), pitch, rows * pitch};
-  at += triple_bytes(rows, pitch);
-  return t;
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(to + i * M::kPart) = a[i];
 }
 
-// Fragments of m16n8k16 in three parts.  rows: stored [m][k] (first operand) or [n][k] (second); turned: [k][m] or [k][n].
-// A second operand's fragment covers 16 columns: words 0, 1 are the first eight, 2, 3 the others.
+// Fragments of m16n8k16 in three parts.  rows: stored [m][k] (first operand) or [n][k] (second), walked along k by
+// 16-column steps; turned: [k][m] or [k][n], walked by rows.  A second operand's fragment covers 16 columns: words 0, 1 are
+// the first eight, 2, 3 the others.
 using Fragment = uint32_t[3][4];
 template <class M>
-__device__ __forceinline__ void first_rows(Fragment& f, const M& m, int row0, int k0, int lane) {
-  const __nv_bfloat16* p = m.p + m.at(row0 + (lane & 15), k0 + (lane >> 4) * 8);
+struct AlongRows {  // the lane's place in rows row0 .. row0 + 15, column 0
+  const __nv_bfloat16* p;
+  int at;
+  __device__ __forceinline__ void load(Fragment& f, int step) const {
+    const __nv_bfloat16* q = p + (at ^ (16 * step));
 #pragma unroll
-  for (int i = 0; i < 3; ++i) load_matrices(f[i], p + i * m.part);
+    for (int i = 0; i < 3; ++i) load_matrices(f[i], q + i * M::kPart);
+  }
+};
+template <class M>
+__device__ __forceinline__ AlongRows<M> first_rows(const M& m, int row0, int lane) { return {m.p, M::at(row0 + (lane & 15), (lane >> 4) * 8)}; }
+template <class M>
+__device__ __forceinline__ AlongRows<M> second_rows(const M& m, int col0, int lane) {
+  return {m.p, M::at(col0 + (lane & 7) + (lane >> 4) * 8, ((lane >> 3) & 1) * 8)};
 }
 template <class M>
-__device__ __forceinline__ void first_turned(Fragment& f, const M& m, int row0, int k0, int lane) {
-  const __nv_bfloat16* p = m.p + m.at(k0 + (lane & 7) + (lane >> 4) * 8, row0 + ((lane >> 3) & 1) * 8);
+struct DownRows {  // the lane's place in rows 0 .. 15
+  const __nv_bfloat16* p;
+  __device__ __forceinline__ void load(Fragment& f, int step) const {
 #pragma unroll
-  for (int i = 0; i < 3; ++i) load_matrices_turned(f[i], p + i * m.part);
+    for (int i = 0; i < 3; ++i) load_matrices_turned(f[i], p + 16 * step * M::kPitch + i * M::kPart);
+  }
+};
+template <class M>
+__device__ __forceinline__ DownRows<M> first_turned(const M& m, int row0, int lane) {
+  return {m.p + M::at((lane & 7) + (lane >> 4) * 8, row0 + ((lane >> 3) & 1) * 8)};
 }
 template <class M>
-__device__ __forceinline__ void second_rows(Fragment& f, const M& m, int col0, int k0, int lane) {
-  const __nv_bfloat16* p = m.p + m.at(col0 + (lane & 7) + (lane >> 4) * 8, k0 + ((lane >> 3) & 1) * 8);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) load_matrices(f[i], p + i * m.part);
-}
-template <class M>
-__device__ __forceinline__ void second_turned(Fragment& f, const M& m, int col0, int k0, int lane) {
-  const __nv_bfloat16* p = m.p + m.at(k0 + (lane & 15), col0 + (lane >> 4) * 8);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) load_matrices_turned(f[i], p + i * m.part);
-}
+__device__ __forceinline__ DownRows<M> second_turned(const M& m, int col0, int lane) { return {m.p + M::at(lane & 15, col0 + (lane >> 4) * 8)}; }
 
 // 16 x 16 results: the high x high products and the five smaller ones apart.
 struct Tile {
@@ -148,19 +158,37 @@ struct Tile {
 };
 
 // The decays of a chunk and what its tokens' writes are multiplied by.  Tokens past the chunk's end: decay 1, factor 0.
-struct Decays {
+struct alignas(16) Decays {
   float g[kChunk], factor[kChunk];
   float pre[kChunk], suf[kChunk];      // within the token's block of 16: the product up to it, and behind it
   float from_start[kChunk], to_end[kChunk];
   float inside[kBlocks][16][17];       // G(i, j) of two tokens of one block
-  __device__ __forceinline__ float between(int i, int j) const {  // G(i, j), i >= j
-    const int bi = i >> 4, bj = j >> 4;
-    if (bi == bj) return inside[bi][i & 15][j & 15];
-    float d = suf[j];
-    for (int b = bj + 1; b < bi; ++b) d *= pre[16 * b + 15];
-    return d * pre[i];
+  // The product of all decays of the blocks between bi and bj < bi: G(i, j) = suf[j] * blocks(bi, bj) * pre[i].
+  __device__ __forceinline__ float blocks(int bi, int bj) const {
+    float x = 1.f;
+    for (int b = bj + 1; b < bi; ++b) x *= pre[16 * b + 15];
+    return x;
   }
 };
+
+// The elements of a 16 x 16 result (rows of block bi, columns of block bj, bi >= bj) times G(i, j); zeros above the diagonal.
+__device__ __forceinline__ void times_decays(float (&x)[2][4], const Tile& t, const Decays& d, int bi, int bj, int lane) {
+  const int g = lane >> 2, c = lane & 3;
+  if (bi == bj) {
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) x[n][r] = t.of(n, r) * d.inside[bi][g + 8 * (r >> 1)][8 * n + 2 * c + (r & 1)];
+  } else {
+    const float mid = d.blocks(bi, bj), up[2] = {d.pre[16 * bi + g] * mid, d.pre[16 * bi + g + 8] * mid};
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      const float2 down = *reinterpret_cast<const float2*>(&d.suf[16 * bj + 8 * n + 2 * c]);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) x[n][r] = t.of(n, r) * (up[r >> 1] * (r & 1 ? down.y : down.x));
+    }
+  }
+}
 
 // Every thread of the block calls it; it ends with a barrier.
 __device__ __forceinline__ void make_decays(Decays& d, const ChunkArgs& a, int rule, int head, int t0, int rows) {
@@ -215,47 +243,50 @@ __device__ __forceinline__ float4 four_at(const float* p, int col, int dim, bool
   return make_float4(p[col], col + 1 < dim ? p[col + 1] : 0.f, col + 2 < dim ? p[col + 2] : 0.f, col + 3 < dim ? p[col + 3] : 0.f);
 }
 
-// N rows of a matrix a warp, four elements a lane (from column 4 lane + offset on): fetched first, stored as parts later, so
-// that the loads of several matrices are in flight together.  Row i of warp w is w + i * WARPS; rows from `live` on and
-// elements from `dim` on are zeros, except that with `unit` element `dim` of a live row is 1.
-template <int N, int WARPS>
+// COUNT rows of a matrix, a warp a row and four elements a lane (from column 4 lane + offset on): fetched first, stored
+// as parts later, so that the loads of several matrices are in flight together.  Rows from `live` on and elements from
+// `dim` on are zeros, except that with `unit` element `dim` of a live row is 1.
+template <int COUNT, int THREADS>
 struct Rows {
-  float4 x[N];
+  static constexpr int LANES = 32, kStep = THREADS / LANES, kMine = (COUNT + kStep - 1) / kStep;
+  float4 x[kMine];
+  static __device__ __forceinline__ int row(int i) { return (int)threadIdx.x / LANES + i * kStep; }
+  static __device__ __forceinline__ int column(int offset) { return 4 * ((int)threadIdx.x % LANES) + offset; }
   __device__ __forceinline__ void fetch(const float* src, int stride, int live, int dim, int offset = 0) {
-    const int c = 4 * (threadIdx.x & 31) + offset, warp = threadIdx.x >> 5;
+    const int c = column(offset);
     const bool fours = by_fours(src, stride, dim);
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
+    for (int i = 0; i < kMine; ++i) {
       x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      const int r = warp + i * WARPS;
-      if (r < live && c < dim) x[i] = four_at(src + (size_t)r * stride, c, dim, fours);
+      if (row(i) < live && c < dim) x[i] = four_at(src + (size_t)row(i) * stride, c, dim, fours);
     }
   }
   // From the slices of 16 columns that chunk_walk leaves.
   __device__ __forceinline__ void fetch_slices(const float* src, int padded, int offset = 0) {
-    const int c = 4 * (threadIdx.x & 31) + offset, warp = threadIdx.x >> 5;
+    const int c = column(offset);
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
+    for (int i = 0; i < kMine; ++i) {
       x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (c < padded) x[i] = *reinterpret_cast<const float4*>(src + ((size_t)(c >> 4) * kChunk + warp + i * WARPS) * 16 + (c & 15));
+      if (c < padded) x[i] = *reinterpret_cast<const float4*>(src + ((size_t)(c >> 4) * kChunk + row(i)) * 16 + (c & 15));
     }
   }
   // Rows of at most 128 elements made unit vectors, times `scale`.
   __device__ __forceinline__ void make_unit(float scale) {
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
+    for (int i = 0; i < kMine; ++i) {
       const float s = scale / sqrtf(warp_sum(x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w) + 1e-6f);
       x[i] = make_float4(x[i].x * s, x[i].y * s, x[i].z * s, x[i].w * s);
     }
   }
   // weight: per row, or null
-  __device__ __forceinline__ void store(const Triple& m, int count, int live, int dim, int padded, const float* weight, bool unit,
+  template <class M>
+  __device__ __forceinline__ void store(const M& m, int count, int live, int dim, int padded, const float* weight, bool unit,
                                         int offset = 0) {
-    const int c = 4 * (threadIdx.x & 31) + offset, warp = threadIdx.x >> 5;
+    const int c = column(offset);
     if (c >= padded) return;
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const int r = warp + i * WARPS;
+    for (int i = 0; i < kMine; ++i) {
+      const int r = row(i);
       if (r >= count) break;
       if (unit && r < live) {
         if (c == dim) x[i].x = 1.f;
@@ -269,20 +300,21 @@ struct Rows {
   }
 };
 
-// N^T [value_dim, key_dim] of a chunk: rows are value elements (U^T is the first operand), columns key elements.
-template <int RULE>
-__global__ void __launch_bounds__(kNarrowThreads, 2) chunk_write_kernel(ChunkArgs a) {
+// N^T [value_dim, key_dim] of a chunk: rows are value elements (U^T is the first operand), columns key elements.  VALUES:
+// columns of U in shared memory (value_dim up to 128, or to 144).
+template <int RULE, int VALUES>
+__global__ void __launch_bounds__(kChunkThreads, VALUES > 128 ? 1 : 2) chunk_write_kernel(ChunkArgs a) {
   extern __shared__ __align__(128) unsigned char chunk_s[];
   __shared__ Decays d;
   int t0;
   const int head = blockIdx.x, rows = chunk_rows(a.q_tiles, blockIdx.y, t0);
   if (rows <= 0) return;
-  unsigned char* at = chunk_s;
-  const Triple k = triple_at(at, kChunk, kKeyPitch), u = triple_at(at, kChunk, value_pitch(a.value_dim));
+  using ValueTriple = Triple<VALUES, kChunk>;
+  const KeyTriple k{reinterpret_cast<__nv_bfloat16*>(chunk_s)};
+  const ValueTriple u{reinterpret_cast<__nv_bfloat16*>(chunk_s + KeyTriple::kBytes)};
   const int group = head / (a.heads / a.groups);
-  constexpr int kWarps = kNarrowThreads / 32;
   const float* v_rows = a.v + (size_t)t0 * a.v_stride + (size_t)head * a.v_dim;
-  Rows<kChunk / kWarps, kWarps> fetched_k, fetched_u;
+  Rows<kChunk, kChunkThreads> fetched_k, fetched_u;
   fetched_k.fetch(a.k + (size_t)t0 * a.k_stride + group * a.key_dim, a.k_stride, rows, a.key_dim);
   fetched_u.fetch(v_rows, a.v_stride, rows, a.v_dim);
   make_decays(d, a, RULE, head, t0, rows);
@@ -293,7 +325,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) chunk_write_kernel(ChunkArg
   const bool unit_column = a.v_dim < a.value_dim;
   fetched_k.store(k, kChunk, rows, a.key_dim, key_padded, nullptr, false);
   fetched_u.store(u, kChunk, rows, a.v_dim, value_padded, d.factor, unit_column);
-  if (value_padded > 128) {
+  if (VALUES > 128) {
     fetched_u.fetch(v_rows, a.v_stride, rows, a.v_dim, 128);
     fetched_u.store(u, kChunk, rows, a.v_dim, value_padded, d.factor, unit_column, 128);
   }
@@ -303,17 +335,19 @@ __global__ void __launch_bounds__(kNarrowThreads, 2) chunk_write_kernel(ChunkArg
   const int m_tiles = value_padded / 16, n_pairs = (key_padded + 31) / 32, steps = (rows + 15) / 16;
   float* dst = a.chunks + ((size_t)blockIdx.y * a.heads + head) * a.value_dim * a.key_dim;
   const bool pairs = (a.key_dim & 1) == 0;
-  for (int unit = warp; unit < m_tiles * n_pairs; unit += kWarps) {  // 16 value by 32 key elements
+  for (int unit = warp; unit < m_tiles * n_pairs; unit += kChunkWarps) {  // 16 value by 32 key elements
     const int m0 = unit % m_tiles * 16, n0 = unit / m_tiles * 32;
     const bool both = n0 + 16 < key_padded;
+    const auto u_at = first_turned(u, m0, lane);
+    const auto k_at = second_turned(k, n0, lane), k_next = second_turned(k, n0 + 16, lane);
     Tile acc[2];
     for (int s = 0; s < steps; ++s) {
       Fragment x, y;
-      first_turned(x, u, m0, 16 * s, lane);
-      second_turned(y, k, n0, 16 * s, lane);
+      u_at.load(x, s);
+      k_at.load(y, s);
       acc[0].add(x, y);
       if (both) {
-        second_turned(y, k, n0 + 16, 16 * s, lane);
+        k_next.load(y, s);
         acc[1].add(x, y);
       }
     }
@@ -380,10 +414,11 @@ __global__ void __launch_bounds__(kChainThreads) chunk_chain_kernel(ChunkArgs a)
 
 // The inverse T of 1 + A, A [64, 64] strictly below the diagonal, both with rows of kSolvePitch floats; T arrives as zeros.
 // Blocks of 16 by substitution, a thread a column; then pairs of blocks, then the pair of pairs:
-// [1 + A11, 0; A21, 1 + A22] has the inverse [T11, 0; -T22 A21 T11, T22].  m_s: 32 x 33 floats.  512 threads.
+// [1 + A11, 0; A21, 1 + A22] has the inverse [T11, 0; -T22 A21 T11, T22].  m_s: 32 x 33 floats.
 constexpr int kSolvePitch = 68;
 __device__ __forceinline__ void invert(const float* A, float* T, float* m_s) {
   const int tid = threadIdx.x;
+  static_assert(kChunkThreads == 256, "threads are shared out by hand");
   if (tid < kChunk) {
     const int b0 = tid & ~15, j = tid & 15;
     float x[16];
@@ -397,44 +432,54 @@ __device__ __forceinline__ void invert(const float* A, float* T, float* m_s) {
     }
   }
   __syncthreads();
-  {
-    const int r0 = (tid >> 8) * 32, i = (tid >> 4) & 15, l = tid & 15;
-    float sum = 0.f;
+  {  // rows 16 + i of both pairs
+    const int i = tid >> 4, l = tid & 15;
+    float sum[2] = {0.f, 0.f};
 #pragma unroll
-    for (int m = 0; m < 16; ++m) sum += A[(r0 + 16 + i) * kSolvePitch + r0 + m] * T[(r0 + m) * kSolvePitch + r0 + l];
-    m_s[tid] = sum;
+    for (int m = 0; m < 16; ++m)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) sum[p] += A[(32 * p + 16 + i) * kSolvePitch + 32 * p + m] * T[(32 * p + m) * kSolvePitch + 32 * p + l];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) m_s[(16 * p + i) * 16 + l] = sum[p];
     __syncthreads();
-    sum = 0.f;
+    sum[0] = sum[1] = 0.f;
 #pragma unroll
-    for (int m = 0; m < 16; ++m) sum += T[(r0 + 16 + i) * kSolvePitch + r0 + 16 + m] * m_s[(tid & 256) + 16 * m + l];
-    T[(r0 + 16 + i) * kSolvePitch + r0 + l] = -sum;
+    for (int m = 0; m < 16; ++m)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) sum[p] += T[(32 * p + 16 + i) * kSolvePitch + 32 * p + 16 + m] * m_s[(16 * p + m) * 16 + l];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) T[(32 * p + 16 + i) * kSolvePitch + 32 * p + l] = -sum[p];
   }
   __syncthreads();
-  const int i = tid >> 5, l = tid & 31;
-  float sum[2] = {0.f, 0.f};
+  const int i = tid >> 5, l = tid & 31;  // rows i, i + 8, i + 16, i + 24
+  float sum[4] = {};
 #pragma unroll 8
   for (int m = 0; m < 32; ++m) {
     const float t = T[m * kSolvePitch + l];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) sum[h] += A[(32 + i + 16 * h) * kSolvePitch + m] * t;
+    for (int h = 0; h < 4; ++h) sum[h] += A[(32 + i + 8 * h) * kSolvePitch + m] * t;
   }
 #pragma unroll
-  for (int h = 0; h < 2; ++h) m_s[(i + 16 * h) * 33 + l] = sum[h];
+  for (int h = 0; h < 4; ++h) m_s[(i + 8 * h) * 33 + l] = sum[h];
   __syncthreads();
-  sum[0] = sum[1] = 0.f;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) sum[h] = 0.f;
 #pragma unroll 8
   for (int m = 0; m < 32; ++m) {
     const float x = m_s[m * 33 + l];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) sum[h] += T[(32 + i + 16 * h) * kSolvePitch + 32 + m] * x;
+    for (int h = 0; h < 4; ++h) sum[h] += T[(32 + i + 8 * h) * kSolvePitch + 32 + m] * x;
   }
 #pragma unroll
-  for (int h = 0; h < 2; ++h) T[(32 + i + 16 * h) * kSolvePitch + l] = -sum[h];
+  for (int h = 0; h < 4; ++h) T[(32 + i + 8 * h) * kSolvePitch + l] = -sum[h];
   __syncthreads();
 }
 
-// What the delta rule's chunk needs besides the state: T, W and K' (images), U_0.
-__global__ void __launch_bounds__(kWideThreads, 1) chunk_solve_kernel(ChunkArgs a) {
+// What the delta rule's chunk needs besides the state: T, W and K' (images), U_0.  Shared memory: K as parts (then, with
+// the place of A and T, b V), A and T as floats, T as parts.
+constexpr size_t kSolveShared = KeyTriple::kBytes + 2 * (size_t)kChunk * kSolvePitch * 4 + SquareTriple::kBytes;
+static_assert(Triple<192, kChunk>::kBytes <= KeyTriple::kBytes + 2 * (size_t)kChunk * kSolvePitch * 4, "V in the place of K, A and T");
+__global__ void __launch_bounds__(kChunkThreads, 2) chunk_solve_kernel(ChunkArgs a) {
   extern __shared__ __align__(128) unsigned char chunk_s[];
   __shared__ Decays d;
   int t0;
@@ -442,125 +487,142 @@ __global__ void __launch_bounds__(kWideThreads, 1) chunk_solve_kernel(ChunkArgs 
   if (rows <= 0) return;
   const int key_padded = up16(a.key_dim), value_padded = up16(a.value_dim), group = head / (a.heads / a.groups);
   unsigned char* at = chunk_s;
-  const Triple k = triple_at(at, kChunk, kKeyPitch), v = triple_at(at, kChunk, value_pitch(a.value_dim));
-  const Triple t_keys = triple_at(at, kChunk, kChunk), t_values = triple_at(at, kChunk, kChunk);
+  const KeyTriple k{reinterpret_cast<__nv_bfloat16*>(at)};
+  const Triple<192, kChunk> v{k.p};
+  at += KeyTriple::kBytes;
   float* A = reinterpret_cast<float*>(at);
-  float *T = A + kChunk * kSolvePitch, *m_s = T + kChunk * kSolvePitch;
+  float* T = A + kChunk * kSolvePitch;
+  at += 2 * kChunk * kSolvePitch * sizeof(float);
+  float* m_s = reinterpret_cast<float*>(at);
+  const SquareTriple t_s{reinterpret_cast<__nv_bfloat16*>(at)};
   const size_t chunk_head = (size_t)blockIdx.y * a.heads + head;
-  const Triple w_image{a.images + 2 * chunk_head * kImage, kKeyPitch, kChunk * kKeyPitch};
-  const Triple k_image{a.images + (2 * chunk_head + 1) * kImage, kKeyPitch, kChunk * kKeyPitch};
+  const KeyTriple w_image{a.images + 2 * chunk_head * kImage};
+  const KeyTriple k_image{a.images + (2 * chunk_head + 1) * kImage};
   float* writes = a.writes + chunk_head * value_padded * kChunk;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
 
-  constexpr int kWarps = kWideThreads / 32;
   const float* v_rows = a.v + (size_t)t0 * a.v_stride + (size_t)head * a.v_dim;
-  Rows<kChunk / kWarps, kWarps> fetched_k, fetched_v;
-  fetched_k.fetch(a.k + (size_t)t0 * a.k_stride + group * a.key_dim, a.k_stride, rows, a.key_dim);
-  fetched_v.fetch(v_rows, a.v_stride, rows, a.v_dim);
-  for (int i = threadIdx.x; i < 2 * kChunk * kSolvePitch; i += kWideThreads) A[i] = 0.f;
+  Rows<kChunk, kChunkThreads> fetched;
+  fetched.fetch(a.k + (size_t)t0 * a.k_stride + group * a.key_dim, a.k_stride, rows, a.key_dim);
+  for (int i = threadIdx.x; i < 2 * kChunk * kSolvePitch; i += kChunkThreads) A[i] = 0.f;
   make_decays(d, a, kRuleDelta, head, t0, rows);
   if (threadIdx.x == 0) a.whole[chunk_head] = d.from_start[kChunk - 1];
-  fetched_k.make_unit(1.f);
-  fetched_k.store(k, kChunk, rows, a.key_dim, key_padded, nullptr, false);
-  fetched_k.store(k_image, kChunk, rows, a.key_dim, key_padded, d.to_end, false);
-  fetched_v.store(v, kChunk, rows, a.v_dim, value_padded, nullptr, false);
-  if (value_padded > 128) {
-    fetched_v.fetch(v_rows, a.v_stride, rows, a.v_dim, 128);
-    fetched_v.store(v, kChunk, rows, a.v_dim, value_padded, nullptr, false, 128);
-  }
+  fetched.make_unit(1.f);
+  fetched.store(k, kChunk, rows, a.key_dim, key_padded, nullptr, false);
+  fetched.store(k_image, kChunk, rows, a.key_dim, key_padded, d.to_end, false);
   __syncthreads();
 
-  if (warp < 10) {  // the blocks of 16 x 16 on and below the diagonal
-    const int bi = warp < 1 ? 0 : warp < 3 ? 1 : warp < 6 ? 2 : 3, bj = warp - bi * (bi + 1) / 2;
+  for (int block = warp; block < 10; block += kChunkWarps) {  // the blocks of 16 x 16 on and below the diagonal
+    const int bi = block < 1 ? 0 : block < 3 ? 1 : block < 6 ? 2 : 3, bj = block - bi * (bi + 1) / 2;
+    const auto x_at = first_rows(k, bi * 16, lane), y_at = second_rows(k, bj * 16, lane);
     Tile acc;
     for (int s = 0; s < key_padded / 16; ++s) {
       Fragment x, y;
-      first_rows(x, k, bi * 16, 16 * s, lane);
-      second_rows(y, k, bj * 16, 16 * s, lane);
+      x_at.load(x, s);
+      y_at.load(y, s);
       acc.add(x, y);
     }
+    float made[2][4];
+    times_decays(made, acc, d, bi, bj, lane);
 #pragma unroll
     for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const int i = bi * 16 + g + 8 * (r >> 1), j = bj * 16 + 8 * n + 2 * c + (r & 1);
-        if (j < i) A[i * kSolvePitch + j] = d.factor[i] * d.between(i, j) * acc.of(n, r);
+        if (j < i) A[i * kSolvePitch + j] = d.factor[i] * made[n][r];
       }
   }
   __syncthreads();
   invert(A, T, m_s);
-  for (int idx = threadIdx.x; idx < kChunk * kChunk / 2; idx += kWideThreads) {
-    const int i = idx / (kChunk / 2), j = 2 * (idx % (kChunk / 2));
-    const float x = T[i * kSolvePitch + j] * d.factor[j], y = T[i * kSolvePitch + j + 1] * d.factor[j + 1];
-    put2(t_values, i, j, x, y);
-    put2(t_keys, i, j, x * d.from_start[j], y * d.from_start[j + 1]);
-  }
-  __syncthreads();
-
-  // Rows of 16 tokens see up to 16 (row + 1) of them: a warp takes an early and a late one.
-  for (int unit = warp & 7; unit < value_padded / 16 || unit < key_padded / 16; unit += 8) {
+  // Rows of 16 tokens see up to 16 (row + 1) of them: a warp takes all four, for the columns of its units.
+  auto times = [&](const auto& m, int unit, Tile (&acc)[4]) {
+    const auto y_at = second_turned(m, unit * 16, lane);
 #pragma unroll
-    for (int which = 0; which < 2; ++which) {
-      const int mt = which ? 3 - (warp >> 3) : warp >> 3;
-      Tile keys, values;
-      for (int s = 0; s <= mt; ++s) {
-        Fragment x, y;
-        if (unit < key_padded / 16) {
-          first_rows(x, t_keys, mt * 16, 16 * s, lane);
-          second_turned(y, k, unit * 16, 16 * s, lane);
-          keys.add(x, y);
-        }
-        if (unit < value_padded / 16) {
-          first_rows(x, t_values, mt * 16, 16 * s, lane);
-          second_turned(y, v, unit * 16, 16 * s, lane);
-          values.add(x, y);
-        }
+    for (int s = 0; s < 4; ++s) {
+      Fragment x, y;
+      y_at.load(y, s);
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) {
+        if (mt < s) continue;
+        first_rows(t_s, mt * 16, lane).load(x, s);
+        acc[mt].add(x, y);
       }
+    }
+  };
+  auto weigh = [&](bool from_start) {
+    for (int idx = threadIdx.x; idx < kChunk * kChunk / 2; idx += kChunkThreads) {
+      const int i = idx / (kChunk / 2), j = 2 * (idx % (kChunk / 2));
+      const float x = T[i * kSolvePitch + j] * d.factor[j], y = T[i * kSolvePitch + j + 1] * d.factor[j + 1];
+      put2(t_s, i, j, from_start ? x * d.from_start[j] : x, from_start ? y * d.from_start[j + 1] : y);
+    }
+  };
+  weigh(true);
+  __syncthreads();
+  fetched.fetch(v_rows, a.v_stride, rows, a.v_dim);
+  for (int unit = warp; unit < key_padded / 16; unit += kChunkWarps) {
+    Tile acc[4];
+    times(k, unit, acc);
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int row = mt * 16 + g + 8 * h, col = 8 * n + 2 * c;
-          if (unit < key_padded / 16) put2(w_image, row, unit * 16 + col, keys.of(n, 2 * h), keys.of(n, 2 * h + 1));
-          if (unit < value_padded / 16)
-            *reinterpret_cast<float2*>(writes + ((size_t)unit * kChunk + row) * 16 + col) =
-                make_float2(values.of(n, 2 * h), values.of(n, 2 * h + 1));
-        }
-    }
+        for (int h = 0; h < 2; ++h)
+          put2(w_image, mt * 16 + g + 8 * h, unit * 16 + 8 * n + 2 * c, acc[mt].of(n, 2 * h), acc[mt].of(n, 2 * h + 1));
+  }
+  __syncthreads();
+  weigh(false);
+  __syncthreads();  // T is in parts, K done with
+  fetched.store(v, kChunk, rows, a.v_dim, value_padded, nullptr, false);
+  if (value_padded > 128) {
+    fetched.fetch(v_rows, a.v_stride, rows, a.v_dim, 128);
+    fetched.store(v, kChunk, rows, a.v_dim, value_padded, nullptr, false, 128);
+  }
+  __syncthreads();
+  for (int unit = warp; unit < value_padded / 16; unit += kChunkWarps) {
+    Tile acc[4];
+    times(v, unit, acc);
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          *reinterpret_cast<float2*>(writes + ((size_t)unit * kChunk + mt * 16 + g + 8 * h) * 16 + 8 * n + 2 * c) =
+              make_float2(acc[mt].of(n, 2 * h), acc[mt].of(n, 2 * h + 1));
   }
 }
 
-// The chain of the delta rule: 16 value elements of one head's state, chunk after chunk.  What it reads of a chunk (W, K'
-// and its slice of U_0: 100 KB) is copied a chunk ahead.  A block whose tile is not the first of its request has nothing
-// to do.
-constexpr int kWalkThreads = 256;
-constexpr size_t kWalkStage = 2 * (size_t)kImage * 2 + kChunk * 16 * 4;
-constexpr size_t kWalkShared = 2 * kWalkStage + triple_bytes(16, kKeyPitch) + (size_t)3 * kChunk * NarrowTriple::kPitch * 2 + 4096;
-__device__ __forceinline__ void copy_16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+// The chain of the delta rule: 16 value elements of one head's state, chunk after chunk.  What it reads of a chunk (W and
+// K', 96 KB) is copied a chunk ahead.  Sixteen warps: in the first product four share the 16 tokens of a row of tiles, each
+// a quarter of the keys, and finish a quarter of the result each; in the second one each owns eight keys of the state.  A
+// block whose tile is not the first of its request has nothing to do.  STEPS: key_dim / 16 rounded up, 0: any.
+constexpr int kWalkThreads = 512;
+constexpr size_t kWalkStage = 2 * (size_t)kImage * 2;
+constexpr size_t kWalkShared = 2 * kWalkStage + 16 + Triple<kKeyPitch, 16>::kBytes + NarrowTriple<kChunk>::kBytes + 16 * 3 * 32 * 8;
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
+template <int STEPS>
 __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(ChunkArgs a) {
   extern __shared__ __align__(128) unsigned char chunk_s[];
   const int slice = blockIdx.x, head = blockIdx.y, tile0 = blockIdx.z, tid = threadIdx.x;
   const int seq = a.token_seq[a.q_tiles[2 * tile0]];
   if (tile0 > 0 && a.token_seq[a.q_tiles[2 * (tile0 - 1)]] == seq) return;
-  unsigned char* at = chunk_s + 2 * kWalkStage;
-  const Triple S_s = triple_at(at, 16, kKeyPitch);
-  const NarrowTriple u_s{reinterpret_cast<__nv_bfloat16*>(at), kChunk * NarrowTriple::kPitch};
-  float4* half_s = reinterpret_cast<float4*>(at + (size_t)3 * kChunk * NarrowTriple::kPitch * 2);  // [2][4][32]
-  const int key_padded = up16(a.key_dim), value_padded = up16(a.value_dim), steps = key_padded / 16;
+  uint64_t* full = reinterpret_cast<uint64_t*>(chunk_s + 2 * kWalkStage);  // one a stage
+  unsigned char* at = chunk_s + 2 * kWalkStage + 16;
+  const Triple<kKeyPitch, 16> S_s{reinterpret_cast<__nv_bfloat16*>(at)};
+  const NarrowTriple<kChunk> u_s{reinterpret_cast<__nv_bfloat16*>(at + S_s.kBytes)};
+  float2* quarter_s = reinterpret_cast<float2*>(at + S_s.kBytes + u_s.kBytes);  // [4 to][3 from][4 mt][32]
+  const int key_padded = up16(a.key_dim), value_padded = up16(a.value_dim), steps = STEPS ? STEPS : key_padded / 16;
   const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, c = lane & 3;
-  const int mt = warp & 3, kh = warp >> 2;  // first product: 16 tokens, every other step over the keys
+  const int mt = warp & 3, kq = warp >> 2;
+  const bool owner = warp * 8 < key_padded;  // of keys of the state
 
-  auto copy_chunk = [&](int chunk, int stage) {
-    unsigned char* to = chunk_s + stage * kWalkStage;
-    const size_t chunk_head = (size_t)chunk * a.heads + head;
-    const unsigned char* from = reinterpret_cast<const unsigned char*>(a.images + 2 * chunk_head * kImage);
-#pragma unroll 8
-    for (int i = 0; i < 2 * kImage * 2 / 16 / kWalkThreads; ++i) copy_16(to + 16 * (i * kWalkThreads + tid), from + 16 * (i * kWalkThreads + tid));
-    const float* u0 = a.writes + (chunk_head * value_padded + (size_t)slice * 16) * kChunk;
-    copy_16(to + 2 * (size_t)kImage * 2 + 16 * tid, u0 + 4 * tid);
-    cp_async_commit();
+  auto copy_chunk = [&](int chunk, int stage) {  // one thread; W and K' lie side by side
+    mbar_expect_tx(&full[stage], (uint32_t)kWalkStage);
+    bulk_load(chunk_s + stage * kWalkStage, a.images + 2 * ((size_t)chunk * a.heads + head) * kImage, (uint32_t)kWalkStage, &full[stage]);
   };
   auto next_chunk = [&](int chunk) {  // -1: the request ends
     if (!(chunk & 1) && a.q_tiles[chunk + 1] > kChunk) return chunk + 1;
@@ -568,110 +630,144 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(ChunkArgs a
     return tile < a.tiles && a.token_seq[a.q_tiles[2 * tile]] == seq ? 2 * tile : -1;
   };
 
-  copy_chunk(2 * tile0, 0);
-  // the warp's part of S^T: 16 values by 16 keys from 16 warp on
-  float S[2][4];
+  if (tid == 0) {
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    copy_chunk(2 * tile0, 0);
+  }
+  // the warp's part of S^T: 16 values by the 8 keys from 8 warp on
+  float S[4];
   const size_t size = (size_t)a.value_dim * a.key_dim;
   float* slot = a.state + ((size_t)a.seq_seat[seq] * a.heads + head) * size;
   const bool pairs = (a.key_dim & 1) == 0;
-  const int col0 = warp * 16 + 2 * c, row0 = slice * 16 + g;
+  const int col0 = warp * 8 + 2 * c, row0 = slice * 16 + g;
 #pragma unroll
-  for (int n = 0; n < 2; ++n)
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int row = row0 + 8 * (r >> 1), col = col0 + 8 * n + (r & 1);
-      S[n][r] = row < a.value_dim && col < a.key_dim ? slot[(size_t)row * a.key_dim + col] : 0.f;
-    }
+  for (int r = 0; r < 4; ++r) {
+    const int row = row0 + 8 * (r >> 1), col = col0 + (r & 1);
+    S[r] = row < a.value_dim && col < a.key_dim ? slot[(size_t)row * a.key_dim + col] : 0.f;
+  }
   auto store_state = [&](float* to) {
 #pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int row = row0 + 8 * h, col = col0 + 8 * n;
-        if (row >= a.value_dim || col >= a.key_dim) continue;
-        float* p = to + (size_t)row * a.key_dim + col;
-        if (pairs) *reinterpret_cast<float2*>(p) = make_float2(S[n][2 * h], S[n][2 * h + 1]);
-        else {
-          p[0] = S[n][2 * h];
-          if (col + 1 < a.key_dim) p[1] = S[n][2 * h + 1];
-        }
+    for (int h = 0; h < 2; ++h) {
+      const int row = row0 + 8 * h;
+      if (row >= a.value_dim || col0 >= a.key_dim) continue;
+      float* p = to + (size_t)row * a.key_dim + col0;
+      if (pairs) *reinterpret_cast<float2*>(p) = make_float2(S[2 * h], S[2 * h + 1]);
+      else {
+        p[0] = S[2 * h];
+        if (col0 + 1 < a.key_dim) p[1] = S[2 * h + 1];
       }
+    }
   };
   auto share_state = [&]() {
-    if (warp * 16 < key_padded) {
+    if (owner) {
 #pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) put2(S_s, g + 8 * h, col0 + 8 * n, S[n][2 * h], S[n][2 * h + 1]);
+      for (int h = 0; h < 2; ++h) put2(S_s, g + 8 * h, col0, S[2 * h], S[2 * h + 1]);
     }
   };
   share_state();
+  __syncthreads();  // the barriers are there
 
-  int stage = 0;
-  for (int chunk = 2 * tile0; chunk >= 0; stage ^= 1) {
-    const int next = next_chunk(chunk);
+  int next = next_chunk(2 * tile0), after = -1;
+  uint32_t round = 0;
+  for (int chunk = 2 * tile0; chunk >= 0; chunk = next, next = after, ++round) {
+    const int stage = round & 1;
+    if (next >= 0 && tid == 0) copy_chunk(next, stage ^ 1);  // its last readers passed a barrier behind their last product
+    after = next >= 0 ? next_chunk(next) : -1;
     const size_t chunk_head = (size_t)chunk * a.heads + head;
     const float whole = a.whole[chunk_head];
-    if (next >= 0) {  // (the stage's last readers passed a barrier behind their last product)
-      copy_chunk(next, stage ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+    // quarter kq of a 16 x 16 tile: its eight columns from 8 (kq & 1), rows g or g + 8
+    float2* out = reinterpret_cast<float2*>(a.writes + (chunk_head * value_padded + (size_t)slice * 16) * kChunk +
+                                            (mt * 16 + g + 8 * (kq >> 1)) * 16 + 8 * (kq & 1) + 2 * c);
+    const float2 ahead = *out;  // U_0
+    const bool here = mbar_wait(&full[stage], (round >> 1) & 1);
+    if (__syncthreads_or(!here)) {  // (given up: the copies in flight get the same time to land)
+      if (tid == 0) {
+        atomicExch(a.error, 6);
+        if (next >= 0) mbar_wait(&full[stage ^ 1], ((round + 1) >> 1) & 1);
+      }
+      return;
     }
-    __syncthreads();
-    unsigned char* base = chunk_s + stage * kWalkStage;
-    const Triple w{reinterpret_cast<__nv_bfloat16*>(base), kKeyPitch, kChunk * kKeyPitch};
-    const Triple k{reinterpret_cast<__nv_bfloat16*>(base) + kImage, kKeyPitch, kChunk * kKeyPitch};
-    const float* u0 = reinterpret_cast<const float*>(base + 2 * (size_t)kImage * 2);
+    const KeyTriple w{reinterpret_cast<__nv_bfloat16*>(chunk_s + stage * kWalkStage)}, k{w.p + kImage};
+    const auto w_at = first_rows(w, mt * 16, lane);
+    const auto S_at = second_rows(S_s, 0, lane);
     store_state(a.chunks + chunk_head * size);
 
-    Tile sum;
-    for (int s = kh; s < steps; s += 2) {
-      Fragment x, y;
-      first_rows(x, w, mt * 16, 16 * s, lane);
-      second_rows(y, S_s, 0, 16 * s, lane);
-      sum.add(x, y);
-    }
-    // each half of the warps finishes eight columns: the other eight go to its partner
-    half_s[((kh ^ 1) * 4 + mt) * 32 + lane] = kh ? make_float4(sum.of(0, 0), sum.of(0, 1), sum.of(0, 2), sum.of(0, 3))
-                                                : make_float4(sum.of(1, 0), sum.of(1, 1), sum.of(1, 2), sum.of(1, 3));
-    __syncthreads();
     {
-      const float4 other = half_s[(kh * 4 + mt) * 32 + lane];
-      const int row = mt * 16 + g, col = 8 * kh + 2 * c;
-      float* out = a.writes + (chunk_head * value_padded + (size_t)slice * 16) * kChunk;
-      const float2 p = *reinterpret_cast<const float2*>(u0 + row * 16 + col), q = *reinterpret_cast<const float2*>(u0 + (row + 8) * 16 + col);
-      const float2 x = make_float2(p.x - (kh ? sum.of(1, 0) : sum.of(0, 0)) - other.x, p.y - (kh ? sum.of(1, 1) : sum.of(0, 1)) - other.y);
-      const float2 y = make_float2(q.x - (kh ? sum.of(1, 2) : sum.of(0, 2)) - other.z, q.y - (kh ? sum.of(1, 3) : sum.of(0, 3)) - other.w);
-      put2(u_s, row, col, x.x, x.y);
-      put2(u_s, row + 8, col, y.x, y.y);
-      *reinterpret_cast<float2*>(out + row * 16 + col) = x;
-      *reinterpret_cast<float2*>(out + (row + 8) * 16 + col) = y;
+      Tile sum;
+      if (STEPS) {
+#pragma unroll
+        for (int i = 0; i < (STEPS + 3) / 4; ++i) {
+          const int s = kq + 4 * i;
+          if (STEPS % 4 && s >= STEPS) break;
+          Fragment x, y;
+          w_at.load(x, s);
+          S_at.load(y, s);
+          sum.add(x, y);
+        }
+      } else {
+        for (int s = kq; s < steps; s += 4) {
+          Fragment x, y;
+          w_at.load(x, s);
+          S_at.load(y, s);
+          sum.add(x, y);
+        }
+      }
+      float2 own = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 part = make_float2(sum.of(i & 1, 2 * (i >> 1)), sum.of(i & 1, 2 * (i >> 1) + 1));
+        if (i == kq) own = part;
+        else quarter_s[((i * 3 + (kq > i ? kq - 1 : kq)) * 4 + mt) * 32 + lane] = part;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const float2 part = quarter_s[((kq * 3 + i) * 4 + mt) * 32 + lane];
+        own.x += part.x;
+        own.y += part.y;
+      }
+      const float2 u = make_float2(ahead.x - own.x, ahead.y - own.y);
+      put2(u_s, mt * 16 + g + 8 * (kq >> 1), 8 * (kq & 1) + 2 * c, u.x, u.y);
+      *out = u;
     }
     __syncthreads();
-    if (warp * 16 < key_padded) {
-      Tile moved;
+    if (owner) {
+      const auto u_at = first_turned(u_s, 0, lane);
+      float high[4] = {}, rest[2][4] = {};
 #pragma unroll
-      for (int s = 0; s < kChunk / 16; ++s) {
-        Fragment x, y;
-        first_turned(x, u_s, 0, 16 * s, lane);
-        second_turned(y, k, warp * 16, 16 * s, lane);
-        moved.add(x, y);
+      for (int s = 0; s < kChunk / 16; s += 2) {
+        Fragment x0, x1, y;  // y: eight keys, both steps
+        u_at.load(x0, s);
+        u_at.load(x1, s + 1);
+        const __nv_bfloat16* p = k.p + k.at(16 * s + lane, warp * 8);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) load_matrices_turned(y[i], p + i * k.kPart);
+        constexpr int kFirst[5] = {2, 0, 1, 1, 0}, kSecond[5] = {0, 2, 1, 0, 1};
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+          mma_16bit(rest[0], x0[kFirst[i]], y[kSecond[i]][0], y[kSecond[i]][1]);
+          mma_16bit(rest[1], x1[kFirst[i]], y[kSecond[i]][2], y[kSecond[i]][3]);
+        }
+        mma_16bit(high, x0[0], y[0][0], y[0][1]);
+        mma_16bit(high, x1[0], y[0][2], y[0][3]);
       }
 #pragma unroll
-      for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) S[n][r] = fmaf(whole, S[n][r], moved.of(n, r));
+      for (int r = 0; r < 4; ++r) S[r] = fmaf(whole, S[r], high[r] + (rest[0][r] + rest[1][r]));
     }
     share_state();  // (every warp has read the old one: two barriers ago)
-    chunk = next;
-    if (chunk >= 0) __syncthreads();  // this stage's copies may be overwritten from here on
+    if (next >= 0) __syncthreads();  // this stage's copies may be overwritten from here on
   }
   store_state(slot);
 }
 
-// O of a chunk from its own tokens and the state before it.
-template <int RULE>
+// O of a chunk from its own tokens and the state before it.  Shared memory: Q | K | S, then Q | the scores | U.
+using StateTriple = Triple<kKeyPitch, 144>;
+constexpr size_t read_shared(int value_dim) {  // (parts of S and U lie as for 144 values where there are more than 128)
+  return 2 * KeyTriple::kBytes + (value_dim > 128 ? StateTriple::kBytes : Triple<kKeyPitch, 128>::kBytes);
+}
+template <int RULE, int VALUES>
 __global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a) {
   extern __shared__ __align__(128) unsigned char chunk_s[];
   __shared__ Decays d;
@@ -679,28 +775,27 @@ __global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a
   const int head = blockIdx.x, rows = chunk_rows(a.q_tiles, blockIdx.y, t0);
   if (rows <= 0) return;
   const int key_padded = up16(a.key_dim), value_padded = up16(a.value_dim), group = head / (a.heads / a.groups);
-  unsigned char* at = chunk_s;
-  const Triple q = triple_at(at, kChunk, kKeyPitch);
-  unsigned char *behind_q = at;
-  const Triple k = triple_at(at, kChunk, kKeyPitch);
-  unsigned char *behind_k = at;
-  const Triple S = triple_at(at, value_padded, kKeyPitch);
-  // once the products with K and S are made, the scores and U lie in their place
-  const Triple p = triple_at(behind_q, kChunk, kChunk), u = triple_at(behind_k, kChunk, value_pitch(a.value_dim));
+  constexpr int kStateRows = VALUES > 128 ? 144 : 128;
+  using ValueTriple = Triple<VALUES, kChunk>;
+  static_assert(ValueTriple::kBytes <= Triple<kKeyPitch, kStateRows>::kBytes, "U in the place of S");
+  const KeyTriple q{reinterpret_cast<__nv_bfloat16*>(chunk_s)}, k{reinterpret_cast<__nv_bfloat16*>(chunk_s + KeyTriple::kBytes)};
+  const Triple<kKeyPitch, kStateRows> S{reinterpret_cast<__nv_bfloat16*>(chunk_s + 2 * KeyTriple::kBytes)};
+  const SquareTriple p{k.p};
+  const ValueTriple u{S.p};
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
   // 16 rows of the chunk; a quarter of the columns.  Later rows see more keys: each scheduler gets warps of all four.
   const int cq = warp >> 2, rg = (warp + cq) & 3;
   const int row0 = rg * 16 + g;
-
-  constexpr int kWarps = kWideThreads / 32;
   const float* v_rows = a.v + (size_t)t0 * a.v_stride + (size_t)head * a.v_dim;
   const bool unit_column = a.v_dim < a.value_dim;
-  Rows<kChunk / kWarps, kWarps> fetched_q, fetched_k, fetched_u;
+  Rows<kChunk, kWideThreads> fetched_u;
   {
-    Rows<9, kWarps> fetched_S;
+    Rows<kChunk, kWideThreads> fetched_q, fetched_k;
+    Rows<kStateRows, kWideThreads> fetched_S;
     fetched_q.fetch(a.q + (size_t)t0 * a.q_stride + group * a.key_dim, a.q_stride, rows, a.key_dim);
     fetched_k.fetch(a.k + (size_t)t0 * a.k_stride + group * a.key_dim, a.k_stride, rows, a.key_dim);
     fetched_S.fetch(a.chunks + ((size_t)blockIdx.y * a.heads + head) * a.value_dim * a.key_dim, a.key_dim, a.value_dim, a.key_dim);
+    make_decays(d, a, RULE, head, t0, rows);
     if (RULE == kRuleDelta) {
       fetched_q.make_unit(rsqrtf((float)a.key_dim));
       fetched_k.make_unit(1.f);
@@ -709,29 +804,35 @@ __global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a
     fetched_k.store(k, kChunk, rows, a.key_dim, key_padded, nullptr, false);
     fetched_S.store(S, value_padded, a.value_dim, a.key_dim, key_padded, nullptr, false);
   }
-  make_decays(d, a, RULE, head, t0, rows);
+  __syncthreads();
 
   const int steps = key_padded / 16, units = value_padded / 16;  // 16 values a unit
-  constexpr int kUnits = 3;                                       // at most, a warp
-  float o[kUnits][2][4];
-  Tile score;
+  constexpr int kUnits = VALUES > 128 ? 3 : 2;                    // at most, a warp
+  const auto q_at = first_rows(q, rg * 16, lane);
+  float o[kUnits][2][4], score[2][4] = {};
   if (cq <= rg) {  // the warp's keys are not all behind its rows
+    const auto k_at = second_rows(k, cq * 16, lane);
+    Tile acc;
+#pragma unroll 2
     for (int s = 0; s < steps; ++s) {
       Fragment x, y;
-      first_rows(x, q, rg * 16, 16 * s, lane);
-      second_rows(y, k, cq * 16, 16 * s, lane);
-      score.add(x, y);
+      q_at.load(x, s);
+      k_at.load(y, s);
+      acc.add(x, y);
     }
+    times_decays(score, acc, d, rg, cq, lane);
   }
 #pragma unroll
   for (int i = 0; i < kUnits; ++i) {
     const int unit = cq + 4 * i;
     if (unit < units) {
+      const auto S_at = second_rows(S, unit * 16, lane);
       Tile acc;
+#pragma unroll 2
       for (int s = 0; s < steps; ++s) {
         Fragment x, y;
-        first_rows(x, q, rg * 16, 16 * s, lane);
-        second_rows(y, S, unit * 16, 16 * s, lane);
+        q_at.load(x, s);
+        S_at.load(y, s);
         acc.add(x, y);
       }
 #pragma unroll
@@ -748,13 +849,9 @@ __global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a
 #pragma unroll
   for (int n = 0; n < 2; ++n)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int row = row0 + 8 * h, key = cq * 16 + 8 * n + 2 * c;
-      put2(p, row, key, key <= row ? score.of(n, 2 * h) * d.between(row, key) : 0.f,
-           key + 1 <= row ? score.of(n, 2 * h + 1) * d.between(row, key + 1) : 0.f);
-    }
+    for (int h = 0; h < 2; ++h) put2(p, row0 + 8 * h, cq * 16 + 8 * n + 2 * c, score[n][2 * h], score[n][2 * h + 1]);
   fetched_u.store(u, kChunk, rows, a.v_dim, value_padded, factor, unit_column);
-  if (value_padded > 128) {
+  if (VALUES > 128) {
     if (RULE == kRuleDelta) fetched_u.fetch_slices(writes, value_padded, 128);
     else fetched_u.fetch(v_rows, a.v_stride, rows, a.v_dim, 128);
     fetched_u.store(u, kChunk, rows, a.v_dim, value_padded, factor, unit_column, 128);
@@ -764,15 +861,17 @@ __global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a
   const float skip = (RULE == kRuleSsd && a.skip) ? a.skip[head] : 0.f;
   float* out = a.out + (size_t)t0 * a.out_stride + (size_t)head * a.value_dim;
   const bool pairs = (a.value_dim & 1) == 0 && (a.out_stride & 1) == 0 && ((uintptr_t)a.out & 7) == 0;
+  const auto p_at = first_rows(p, rg * 16, lane);
 #pragma unroll
   for (int i = 0; i < kUnits; ++i) {
     const int unit = cq + 4 * i;
     if (unit >= units) break;
+    const auto u_at = second_turned(u, unit * 16, lane);
     Tile acc;
     for (int s = 0; s <= rg; ++s) {  // keys up to the warp's last row
       Fragment x, y;
-      first_rows(x, p, rg * 16, 16 * s, lane);
-      second_turned(y, u, unit * 16, 16 * s, lane);
+      p_at.load(x, s);
+      u_at.load(y, s);
       acc.add(x, y);
     }
 #pragma unroll
@@ -783,7 +882,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a
         if (row >= rows || col >= a.value_dim) continue;
         float x = o[i][n][2 * h] + acc.of(n, 2 * h), y = o[i][n][2 * h + 1] + acc.of(n, 2 * h + 1);
         if (RULE == kRuleSsd) {
-          const float* v = a.v + (size_t)(t0 + row) * a.v_stride + (size_t)head * a.v_dim + col;
+          const float* v = v_rows + (size_t)row * a.v_stride + col;
           x += skip * v[0];
           if (col + 1 < a.value_dim) y += skip * v[1];
         }
@@ -815,9 +914,9 @@ extern "C" int distie_recurrence_chunks(int rule, const float* q, int q_stride, 
                                         int splits, long long split_stride, const float* rate, const float* bias, const float* skip,
                                         float* state, float* out, int out_stride, float* scratch, const int* q_tiles, int tiles,
                                         const int* token_seq, const int* seq_seat, int heads, int groups, int key_dim, int value_dim,
-                                        int unit_column, cudaStream_t stream) {
+                                        int unit_column, int* error, cudaStream_t stream) {
   if (tiles <= 0) return 0;
-  if (heads < 1 || groups < 1 || heads % groups || key_dim < 1 || value_dim < 1 || splits < 1 || !q_tiles || !scratch || !state ||
+  if (!error || heads < 1 || groups < 1 || heads % groups || key_dim < 1 || value_dim < 1 || splits < 1 || !q_tiles || !scratch || !state ||
       rule < kRuleDelta || rule > kRuleGated || (rule == kRuleDelta && !decay) ||
       (rule != kRuleGated && (!rate || !write || unit_column)) || (rule == kRuleGated && !rate && !decay) ||
       (unit_column && value_dim < 2))
@@ -839,9 +938,9 @@ extern "C" int distie_recurrence_chunks(int rule, const float* q, int q_stride, 
   a.q_tiles = q_tiles; a.token_seq = token_seq; a.seq_seat = seq_seat;
   a.tiles = tiles; a.heads = heads; a.groups = groups; a.key_dim = key_dim; a.value_dim = value_dim;
   a.v_dim = unit_column ? value_dim - 1 : value_dim;
+  a.error = error;
   const dim3 grid(heads, 2 * tiles);
-  const size_t key_bytes = triple_bytes(kChunk, kKeyPitch), value_bytes = triple_bytes(kChunk, value_pitch(value_dim));
-  const size_t state_bytes = triple_bytes(up16(value_dim), kKeyPitch);
+  const bool narrow = value_dim <= 128;
   auto launch = [&](auto kernel, dim3 blocks, int threads, size_t shared) -> int {
     if (shared > 48 * 1024) {
       cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
@@ -850,18 +949,24 @@ extern "C" int distie_recurrence_chunks(int rule, const float* q, int q_stride, 
     kernel<<<blocks, threads, shared, stream>>>(a);
     return (int)cudaGetLastError();
   };
-  // in chunk_read the scores lie where K was, U where S was: each is taken at the larger of the two
-  const size_t read_shared = 2 * key_bytes + (state_bytes > value_bytes ? state_bytes : value_bytes);
+#define DISTIE_READ(RULE)                                                                              \
+  (narrow ? launch(chunk_read_kernel<RULE, 128>, grid, kWideThreads, read_shared(value_dim))           \
+          : launch(chunk_read_kernel<RULE, 192>, grid, kWideThreads, read_shared(value_dim)))
   int status;
   if (rule == kRuleDelta) {
-    const size_t solve_shared = key_bytes + value_bytes + 2 * triple_bytes(kChunk, kChunk) + (2 * kChunk * kSolvePitch + 32 * 33) * sizeof(float);
-    status = launch(chunk_solve_kernel, grid, kWideThreads, solve_shared);
-    if (status == 0) status = launch(chunk_walk_kernel, dim3(up16(value_dim) / 16, heads, tiles), kWalkThreads, kWalkShared);
-    return status != 0 ? status : launch(chunk_read_kernel<kRuleDelta>, grid, kWideThreads, read_shared);
+    status = launch(chunk_solve_kernel, grid, kChunkThreads, kSolveShared);
+    const dim3 walk(up16(value_dim) / 16, heads, tiles);
+    if (status == 0)
+      status = up16(key_dim) == 128 ? launch(chunk_walk_kernel<8>, walk, kWalkThreads, kWalkShared)
+                                    : launch(chunk_walk_kernel<0>, walk, kWalkThreads, kWalkShared);
+    return status != 0 ? status : DISTIE_READ(kRuleDelta);
   }
-  const size_t write_shared = key_bytes + value_bytes;
-  status = rule == kRuleSsd ? launch(chunk_write_kernel<kRuleSsd>, grid, kNarrowThreads, write_shared)
-                            : launch(chunk_write_kernel<kRuleGated>, grid, kNarrowThreads, write_shared);
+  const size_t write_shared = KeyTriple::kBytes + (narrow ? Triple<128, kChunk>::kBytes : Triple<192, kChunk>::kBytes);
+#define DISTIE_WRITE(RULE)                                                                       \
+  (narrow ? launch(chunk_write_kernel<RULE, 128>, grid, kChunkThreads, write_shared)             \
+          : launch(chunk_write_kernel<RULE, 192>, grid, kChunkThreads, write_shared))
+  status = rule == kRuleSsd ? DISTIE_WRITE(kRuleSsd) : DISTIE_WRITE(kRuleGated);
+#undef DISTIE_WRITE
   if (status != 0) return status;
   const int size = key_dim * value_dim;
   const bool fours = (size & 3) == 0 && ((uintptr_t)state & 15) == 0;
@@ -869,6 +974,7 @@ extern "C" int distie_recurrence_chunks(int rule, const float* q, int q_stride, 
   const dim3 chain((size / width + kChainThreads - 1) / kChainThreads, heads, tiles);
   status = fours ? launch(chunk_chain_kernel<4>, chain, kChainThreads, 0) : launch(chunk_chain_kernel<1>, chain, kChainThreads, 0);
   if (status != 0) return status;
-  return rule == kRuleSsd ? launch(chunk_read_kernel<kRuleSsd>, grid, kWideThreads, read_shared)
-                          : launch(chunk_read_kernel<kRuleGated>, grid, kWideThreads, read_shared);
+  return rule == kRuleSsd ? DISTIE_READ(kRuleSsd)
+                          : DISTIE_READ(kRuleGated);
+#undef DISTIE_READ
 }

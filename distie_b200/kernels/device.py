@@ -651,7 +651,8 @@ class DeviceKernels(KernelSet):
             check(
                 function("distie_recurrence_chunks")(
                     *head, chunks.data_ptr(), step.q_tiles.data_ptr(), step.num_q_tiles, step.token_seq.data_ptr(),
-                    step.seq_seat.data_ptr(), heads, groups, key_dim, value_dim, int(bool(unit_column)), self._stream(),
+                    step.seq_seat.data_ptr(), heads, groups, key_dim, value_dim, int(bool(unit_column)),
+                    self.error_flag.data_ptr(), self._stream(),
                 ),
                 "recurrence_chunks",
             )

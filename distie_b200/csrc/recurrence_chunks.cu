@@ -624,12 +624,15 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(ChunkArgs a
     mbar_expect_tx(&full[stage], (uint32_t)kWalkStage);
     bulk_load(chunk_s + stage * kWalkStage, a.images + 2 * ((size_t)chunk * a.heads + head) * kImage, (uint32_t)kWalkStage, &full[stage]);
   };
-  auto next_chunk = [&](int chunk) {  // -1: the request ends
-    if (!(chunk & 1) && a.q_tiles[chunk + 1] > kChunk) return chunk + 1;
-    const int tile = (chunk >> 1) + 1;
-    return tile < a.tiles && a.token_seq[a.q_tiles[2 * tile]] == seq ? 2 * tile : -1;
-  };
-
+  // The request's tiles follow one another, all but the last of them full: its chunks are a range.
+  int tiles = 0;
+  for (int ahead = 0; tile0 + ahead < a.tiles; ahead += kWalkThreads) {
+    const int tile = tile0 + ahead + tid;
+    const int mine = __syncthreads_count(tile < a.tiles && a.token_seq[a.q_tiles[2 * min(tile, a.tiles - 1)]] == seq);
+    tiles += mine;
+    if (mine < kWalkThreads) break;
+  }
+  const int end = 2 * (tile0 + tiles) - (a.q_tiles[2 * (tile0 + tiles) - 1] <= kChunk);
   if (tid == 0) {
     mbar_init(&full[0], 1);
     mbar_init(&full[1], 1);
@@ -669,30 +672,37 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(ChunkArgs a
   share_state();
   __syncthreads();  // the barriers are there
 
-  int next = next_chunk(2 * tile0), after = -1;
-  uint32_t round = 0;
-  for (int chunk = 2 * tile0; chunk >= 0; chunk = next, next = after, ++round) {
+  // quarter kq of a 16 x 16 tile: its eight columns from 8 (kq & 1), rows g or g + 8
+  float2* out = reinterpret_cast<float2*>(a.writes + (((size_t)2 * tile0 * a.heads + head) * value_padded + (size_t)slice * 16) * kChunk +
+                                          (mt * 16 + g + 8 * (kq >> 1)) * 16 + 8 * (kq & 1) + 2 * c);
+  const size_t out_step = (size_t)a.heads * value_padded * kChunk / 2, chunk_step = (size_t)a.heads * size;
+  float* before = a.chunks + ((size_t)2 * tile0 * a.heads + head) * size;
+  const float* whole_at = a.whole + (size_t)2 * tile0 * a.heads + head;
+  float2 ahead = *out;  // U_0 of the coming chunk
+  float whole = *whole_at;
+  for (int chunk = 2 * tile0, round = 0; chunk < end; ++chunk, ++round) {
     const int stage = round & 1;
-    if (next >= 0 && tid == 0) copy_chunk(next, stage ^ 1);  // its last readers passed a barrier behind their last product
-    after = next >= 0 ? next_chunk(next) : -1;
-    const size_t chunk_head = (size_t)chunk * a.heads + head;
-    const float whole = a.whole[chunk_head];
-    // quarter kq of a 16 x 16 tile: its eight columns from 8 (kq & 1), rows g or g + 8
-    float2* out = reinterpret_cast<float2*>(a.writes + (chunk_head * value_padded + (size_t)slice * 16) * kChunk +
-                                            (mt * 16 + g + 8 * (kq >> 1)) * 16 + 8 * (kq & 1) + 2 * c);
-    const float2 ahead = *out;  // U_0
+    const bool more = chunk + 1 < end;
+    if (more && tid == 0) copy_chunk(chunk + 1, stage ^ 1);  // its last readers passed a barrier behind their last product
+    const float2 u0 = ahead;
+    const float decay = whole;
+    if (more) {
+      ahead = out[out_step];
+      whole = *(whole_at += a.heads);
+    }
     const bool here = mbar_wait(&full[stage], (round >> 1) & 1);
     if (__syncthreads_or(!here)) {  // (given up: the copies in flight get the same time to land)
       if (tid == 0) {
         atomicExch(a.error, 6);
-        if (next >= 0) mbar_wait(&full[stage ^ 1], ((round + 1) >> 1) & 1);
+        if (more) mbar_wait(&full[stage ^ 1], ((round + 1) >> 1) & 1);
       }
       return;
     }
     const KeyTriple w{reinterpret_cast<__nv_bfloat16*>(chunk_s + stage * kWalkStage)}, k{w.p + kImage};
     const auto w_at = first_rows(w, mt * 16, lane);
     const auto S_at = second_rows(S_s, 0, lane);
-    store_state(a.chunks + chunk_head * size);
+    store_state(before);
+    before += chunk_step;
 
     {
       Tile sum;
@@ -728,9 +738,10 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(ChunkArgs a
         own.x += part.x;
         own.y += part.y;
       }
-      const float2 u = make_float2(ahead.x - own.x, ahead.y - own.y);
+      const float2 u = make_float2(u0.x - own.x, u0.y - own.y);
       put2(u_s, mt * 16 + g + 8 * (kq >> 1), 8 * (kq & 1) + 2 * c, u.x, u.y);
       *out = u;
+      out += out_step;
     }
     __syncthreads();
     if (owner) {
@@ -754,10 +765,10 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(ChunkArgs a
         mma_16bit(high, x1[0], y[0][2], y[0][3]);
       }
 #pragma unroll
-      for (int r = 0; r < 4; ++r) S[r] = fmaf(whole, S[r], high[r] + (rest[0][r] + rest[1][r]));
+      for (int r = 0; r < 4; ++r) S[r] = fmaf(decay, S[r], high[r] + (rest[0][r] + rest[1][r]));
     }
     share_state();  // (every warp has read the old one: two barriers ago)
-    if (next >= 0) __syncthreads();  // this stage's copies may be overwritten from here on
+    if (more) __syncthreads();  // this stage's copies may be overwritten from here on
   }
   store_state(slot);
 }

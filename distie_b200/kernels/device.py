@@ -33,6 +33,7 @@ _CLUSTER_SPLITS = 8             # splits of a decode attention that one cluster 
 _TENSOR_CORE_ROWS = 128         # from here on the tcgen05 kernel's 128-row tiles are full; in between: the library
 _MAX_TERMS = 24                 # terms of a pending sum that the layer-norm kernel adds up itself
 _RULES = {"delta": 0, "ssd": 1, "gated": 2}
+_CHUNKS_FROM = {"delta": (110, 500), "ssd": (48, 1700), "gated": (48, 1700)}  # tokens a portion, and tokens times heads a step
 _CHUNK_BYTES = 1 << 30          # the most that the states between the chunks of a step may take
 _ACTS = {"relu2": 1, "gelu": 2, "xielu": 3}
 _SCORINGS = {"sigmoid": 0, "softmax": 1, "softmax_chosen": 2}
@@ -475,19 +476,41 @@ class DeviceKernels(KernelSet):
             )
             self._ran("attention_prefill")
         elif rest > 0:
-            check(
-                function("distie_attention_generic")(
-                    qkv.data_ptr() + n_dec * qkv.stride(0) * element, qkv.stride(0),
-                    out.data_ptr() + n_dec * out.stride(0) * element, out.stride(0),
-                    step.positions.data_ptr() + 4 * n_dec, step.token_seq.data_ptr() + 4 * n_dec,
-                    step.seq_seat.data_ptr(), kv.block_table.data_ptr(), kv.block_table.shape[-1],
-                    kv.k.data_ptr(), kv.v.data_ptr(), rest, num_heads, num_kv_heads, head_dim, value_dim, kv.page_size,
-                    kv.num_pages, window, chunk, keep_first, float(scale), softcap, sink_ptr, self.code,
-                    self.error_flag.data_ptr(), self._stream(),
-                ),
-                "attention_generic",
-            )
-            self._ran("attention_generic")
+            if self._attention_tiles(qkv, out, step, kv, num_heads, num_kv_heads, head_dim, window, chunk, scale, keep_first,
+                                     softcap, sink_ptr):
+                rest = step.num_decode_tokens - n_dec  # single tokens of a size without a decode kernel
+            if rest > 0:
+                check(
+                    function("distie_attention_generic")(
+                        qkv.data_ptr() + n_dec * qkv.stride(0) * element, qkv.stride(0),
+                        out.data_ptr() + n_dec * out.stride(0) * element, out.stride(0),
+                        step.positions.data_ptr() + 4 * n_dec, step.token_seq.data_ptr() + 4 * n_dec,
+                        step.seq_seat.data_ptr(), kv.block_table.data_ptr(), kv.block_table.shape[-1],
+                        kv.k.data_ptr(), kv.v.data_ptr(), rest, num_heads, num_kv_heads, head_dim, value_dim, kv.page_size,
+                        kv.num_pages, window, chunk, keep_first, float(scale), softcap, sink_ptr, self.code,
+                        self.error_flag.data_ptr(), self._stream(),
+                    ),
+                    "attention_generic",
+                )
+                self._ran("attention_generic")
+
+    def _attention_tiles(self, qkv, out, step, kv, num_heads, num_kv_heads, head_dim, window, chunk, scale, keep_first,
+                         softcap, sink_ptr) -> bool:
+        """Portions of the float32 engine on the tiled kernel; False when it refuses a size or an alignment."""
+        if self.dtype != torch.float32 or not step.num_q_tiles:
+            return False
+        code = function("distie_attention_tiles")(
+            qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), step.q_tiles.data_ptr(), step.num_q_tiles,
+            step.positions.data_ptr(), step.token_seq.data_ptr(), step.seq_seat.data_ptr(), kv.block_table.data_ptr(),
+            kv.block_table.shape[-1], kv.k.data_ptr(), kv.v.data_ptr(), num_heads, num_kv_heads, head_dim, kv.v.shape[-1],
+            kv.page_size, kv.num_pages, window, chunk, keep_first, float(scale), float(softcap), sink_ptr,
+            self.error_flag.data_ptr(), self._stream(),
+        )
+        if code == -2:
+            return False
+        check(code, "attention_tiles")
+        self._ran("attention_tiles")
+        return True
 
     def _attention_tcgen05(self, qkv, out, step, kv, num_heads, num_kv_heads, head_dim, window, chunk, scale,
                            keep_first=0, softcap=0.0, sink_ptr=None) -> bool:
@@ -677,12 +700,16 @@ class DeviceKernels(KernelSet):
         The walk takes 0.18 us a token of the longest portion while its columns do not fill the machine, and grows with
         the tokens of the step once they do; the chunks cost about 30 us and then 0.05 us a token and 12 heads.  Measured
         with heads of 128 (walk / chunks, us): one portion, 12 heads, 128 tokens 28 / 33, 192 tokens 40 / 34, 2,048
-        tokens 372 / 98; 28 heads, 96 tokens 31 / 34, 128 tokens 40 / 34; four portions of 64 with 12 heads 27 / 34, of
-        96 38 / 35; sixteen of 33 54 / 65, of 64 92 / 70.  The line below lies between these."""
+        tokens 372 / 92; 28 heads, 96 tokens 31 / 34, 128 tokens 40 / 34; four portions of 64 with 12 heads 27 / 34, of
+        96 38 / 35; sixteen of 33 54 / 65, of 64 92 / 70.  The delta rule's chunks cost more (solving for the writes):
+        one portion, 12 heads, 128 tokens 38 / 41, 192 tokens 53 / 44, 2,048 tokens 507 / 169; 28 heads, 128 tokens
+        47 / 48; four portions of 128 with 12 heads 55 / 55; sixteen of 96 150 / 170, of 128 196 / 171.  The lines of
+        _CHUNKS_FROM lie between these."""
         singles = step.num_decode_tokens
         portions, rest = step.num_seqs - singles, step.num_tokens - singles
         return (self.dtype == torch.bfloat16 and portions > 0 and step.num_q_tiles > 0
-                and rest >= 48 * portions + 1700 / heads and key_dim <= 128 and value_dim <= 144 and state.is_contiguous()
+                and rest >= _CHUNKS_FROM[rule][0] * portions + _CHUNKS_FROM[rule][1] / heads
+                and key_dim <= 128 and value_dim <= 144 and state.is_contiguous()
                 and 4 * function("distie_recurrence_chunks_scratch_floats")(_RULES[rule], step.num_q_tiles, heads, key_dim,
                                                                             value_dim) <= _CHUNK_BYTES)
 

@@ -496,8 +496,14 @@ class DeviceKernels(KernelSet):
 
     def _attention_tiles(self, qkv, out, step, kv, num_heads, num_kv_heads, head_dim, window, chunk, scale, keep_first,
                          softcap, sink_ptr) -> bool:
-        """Portions of the float32 engine on the tiled kernel; False when it refuses a size or an alignment."""
-        if self.dtype != torch.float32 or not step.num_q_tiles:
+        """Portions of the float32 engine on the tiled kernel; False when it refuses a size or an alignment.
+
+        A block of it takes 32 rows and keys 64 at a time, so a few rows over a few keys stay on the size-agnostic kernel:
+        that one takes 0.24 us a key of the longest row and the tiles 7 to 10 us and then 0.1 us a key (12 and 28 heads of
+        128; 8 rows alone: 4.5 against 9.5 us, behind 1,000 keys 241 against 102; 32 rows alone: 10.5 against 10.0;
+        500: 373 against 60)."""
+        rows = step.num_tokens - step.num_decode_tokens
+        if self.dtype != torch.float32 or not step.num_q_tiles or (rows < 32 and step.max_kv_len <= 64):
             return False
         code = function("distie_attention_tiles")(
             qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), step.q_tiles.data_ptr(), step.num_q_tiles,

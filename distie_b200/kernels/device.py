@@ -15,6 +15,7 @@ There is no CPU path here and no fallback: a missing library raises.
 
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 import ctypes
@@ -65,6 +66,7 @@ class DeviceKernels(KernelSet):
         if major != 10:
             raise KernelError(f"kernels are built for sm_100a; device reports sm_{major}{minor}")
         self.code = _CODE[dtype]
+        self._index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         if dtype == torch.float32:
             # True 32-bit products: no TF32, no reduced-precision reductions.
             torch.backends.cuda.matmul.allow_tf32 = False
@@ -79,9 +81,9 @@ class DeviceKernels(KernelSet):
         self.kernel_counts: dict[str, int] = {}  # the same, by launcher
 
     # -- helpers ------------------------------------------------------------
-    @staticmethod
-    def _stream() -> int:
-        return torch.cuda.current_stream().cuda_stream
+    def _stream(self) -> int:
+        # The handle alone: torch.cuda.current_stream() builds an object around it, 3 us a launch on the host.
+        return torch._C._cuda_getCurrentRawStream(self._index)
 
     def _ran(self, name: str, kernels: int = 1) -> None:
         self.launches += kernels
@@ -1265,12 +1267,18 @@ class DeviceKernels(KernelSet):
             work += s.q_len * (end - first)
         made = None
         if blocks and work >= _EXPAND_QUERIES * 128 * len(blocks):
-            width = max(b[3] for b in blocks)
-            table = torch.full((len(seqs), -(-width // 128)), -1, dtype=torch.int32)
+            width = -(-max(b[3] for b in blocks) // 128)
+            # One pinned buffer and one copy that nobody waits for; the allocator keeps the buffer until the copy has run.
+            host = torch.empty(4 * len(blocks) + len(seqs) * width, dtype=torch.int32, pin_memory=True)
+            numbers = host.numpy()
+            numbers[: 4 * len(blocks)] = np.asarray(blocks, dtype=np.int32).reshape(-1)
+            table = numbers[4 * len(blocks) :].reshape(len(seqs), width)
+            table[:] = -1
             for row, (first_block, at) in spans.items():
                 count = -(-(seqs[row].past_len + seqs[row].q_len) // 128) - first_block
-                table[row, first_block : first_block + count] = torch.arange(at, at + count, dtype=torch.int32)
-            made = (torch.tensor(blocks, dtype=torch.int32).to(self.device), table.to(self.device), 128 * len(blocks))
+                table[row, first_block : first_block + count] = np.arange(at, at + count, dtype=np.int32)
+            device = host.to(self.device, non_blocking=True)
+            made = (device[: 4 * len(blocks)].view(-1, 4), device[4 * len(blocks) :].view(len(seqs), width), 128 * len(blocks))
         step.derived[key] = made
         return made
 

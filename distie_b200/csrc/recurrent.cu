@@ -792,124 +792,109 @@ __global__ void activation_kernel(Sliced x, T* __restrict__ out, int tokens, int
 // Exponential gates under a running maximum:
 //   i = cap tanh((x_i + b_i) / cap);  f = logsigmoid(cap tanh((x_f + b_f) / cap));  m_t = max(f_t + m_(t-1), i_t)
 //   keep = exp(f + m_(t-1) - m_t);  take = exp(i - m_t);  floor = exp(-m_t);  m lives in state[seat, head].
-// Three kernels.  The gates of all tokens side by side over the whole machine (f into `keep`, i into `take`).  Then
-// a block per request walks its tokens: a tile of gates comes into shared memory, a thread per head runs the chain
-// (an addition and a maximum per token, its operands on the chip; it reads two arrays and writes three others, so
-// that later loads need not wait for earlier stores), and the exponents go back out.  Then the exponentials side
-// by side.  The walk is the plain sequence of operations whatever the tile or the cutting of the prompt.
+// A step of single tokens: one kernel.  Otherwise two, a block per request and chunk of its tokens.  The first makes the
+// gates and what a chunk does to the maximum before it, m -> max(m + F, I) with F the sum of its f and I the maximum it
+// would leave behind nothing; the second finds its chunk's m from the chunks before it, walks its tokens from there in the
+// plain sequence of operations and takes the exponentials.  (One block walking a request's tokens took 31 us for 1,531
+// tokens of 12 heads, with 5 us around it; these two take 8.)
 // ---------------------------------------------------------------------------
-__global__ void exp_gates_kernel(Sliced log_in, Sliced log_forget, const float* __restrict__ in_bias,
-                                 const float* __restrict__ forget_bias, float cap, int tokens, int heads,
-                                 float* __restrict__ keep, float* __restrict__ take) {
-  const size_t total = (size_t)tokens * heads;
-  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
-    const size_t t = idx / heads;
-    const int h = (int)(idx % heads);
-    take[idx] = cap * tanhf((log_in.at(t, h) + in_bias[h]) / cap);
-    keep[idx] = -softplus_f(-(cap * tanhf((log_forget.at(t, h) + forget_bias[h]) / cap)));
+constexpr int kGateThreads = 256;
+__host__ __device__ constexpr int gate_chunk(int heads) { return heads <= 64 ? 64 : 4096 / heads; }  // tokens (512 heads: 8)
+
+struct GateScan {
+  Sliced log_in, log_forget;
+  const float *in_bias, *forget_bias;
+  float cap;
+  float* state;
+  const int *seq_bounds, *seq_seat;
+  int heads, chunk;
+  float *keep, *take, *floor_out;
+  float2* moves;  // [tokens / chunk + requests + 1, heads]: F and I
+  float* before;  // [requests, heads]: m before the step
+  __device__ __forceinline__ float in_gate(size_t t, int h) const { return cap * tanhf((log_in.at(t, h) + in_bias[h]) / cap); }
+  __device__ __forceinline__ float forget_gate(size_t t, int h) const {
+    return -softplus_f(-(cap * tanhf((log_forget.at(t, h) + forget_bias[h]) / cap)));
   }
+  __device__ __forceinline__ float2* moves_of(int row, int first, int index) const {
+    return moves + (size_t)(first / chunk + row + index) * heads;
+  }
+};
+
+__global__ void __launch_bounds__(kGateThreads) exp_gate_single_kernel(GateScan a, int rows) {
+  const int idx = blockIdx.x * kGateThreads + threadIdx.x;
+  if (idx >= rows * a.heads) return;
+  const int row = idx / a.heads, h = idx % a.heads, t = a.seq_bounds[row];
+  if (a.seq_bounds[row + 1] <= t) return;
+  float* slot = a.state + (size_t)a.seq_seat[row] * a.heads + h;
+  const float f = a.forget_gate(t, h), i = a.in_gate(t, h), m = *slot, m_new = fmaxf(f + m, i);
+  const size_t at = (size_t)t * a.heads + h;
+  a.keep[at] = expf(f + m - m_new);
+  a.take[at] = expf(i - m_new);
+  a.floor_out[at] = expf(-m_new);
+  *slot = m_new;
 }
 
-// gates_s: 5 * tile_tokens * heads floats of dynamic shared memory.
-__global__ void __launch_bounds__(512)
-exp_gate_scan_kernel(float* __restrict__ state, const int* __restrict__ seq_bounds, const int* __restrict__ seq_seat,
-                     int heads, int tile_tokens, float* __restrict__ keep, float* __restrict__ take,
-                     float* __restrict__ floor_out) {
+// Dynamic shared memory: 2 * chunk * heads floats.
+__global__ void __launch_bounds__(kGateThreads) exp_gate_moves_kernel(GateScan a) {
   extern __shared__ float gates_s[];
-  const size_t plane = (size_t)tile_tokens * heads;
-  const float* __restrict__ f_in = gates_s;
-  const float* __restrict__ i_in = gates_s + plane;
-  float* __restrict__ keep_o = gates_s + 2 * plane;
-  float* __restrict__ take_o = gates_s + 3 * plane;
-  float* __restrict__ floor_o = gates_s + 4 * plane;
-  const int row = blockIdx.x;
-  const int first = seq_bounds[row], end = seq_bounds[row + 1];
-  float m = 0.f;
-  float* slot = nullptr;
-  if (threadIdx.x < heads) {
-    slot = state + (size_t)seq_seat[row] * heads + threadIdx.x;
-    m = *slot;
+  const int row = blockIdx.y, first = a.seq_bounds[row], t0 = first + blockIdx.x * a.chunk, end = a.seq_bounds[row + 1];
+  if (t0 >= end) return;
+  const int count = min(a.chunk, end - t0) * a.heads, plane = a.chunk * a.heads;
+  for (int idx = threadIdx.x; idx < count; idx += kGateThreads) {
+    const size_t t = t0 + idx / a.heads;
+    const int h = idx % a.heads;
+    const float f = a.forget_gate(t, h), i = a.in_gate(t, h);
+    gates_s[idx] = f;
+    gates_s[plane + idx] = i;
+    a.keep[(size_t)t0 * a.heads + idx] = f;
+    a.take[(size_t)t0 * a.heads + idx] = i;
   }
-  for (int tile = first; tile < end; tile += tile_tokens) {
-    const int count = min(tile_tokens, end - tile) * heads;
-    const size_t base = (size_t)tile * heads;
-    // (16 bytes a thread and round where the tile starts on a 16-byte boundary: all of a thread's loads in flight)
-    const bool quads = (base & 3) == 0 && (count & 3) == 0 && (plane & 3) == 0 &&
-                       (((uintptr_t)keep | (uintptr_t)take | (uintptr_t)floor_out) & 15) == 0;
-    if (quads) {
-#pragma unroll 4
-      for (int idx = threadIdx.x * 4; idx < count; idx += blockDim.x * 4) {
-        *reinterpret_cast<float4*>(gates_s + idx) = *reinterpret_cast<const float4*>(keep + base + idx);
-        *reinterpret_cast<float4*>(gates_s + plane + idx) = *reinterpret_cast<const float4*>(take + base + idx);
-      }
-    } else {
-      for (int idx = threadIdx.x; idx < count; idx += blockDim.x) {
-        gates_s[idx] = keep[base + idx];
-        gates_s[plane + idx] = take[base + idx];
-      }
+  __syncthreads();
+  for (int h = threadIdx.x; h < a.heads; h += kGateThreads) {
+    float sum = 0.f, m = -INFINITY;
+    for (int at = h; at < count; at += a.heads) {
+      sum += gates_s[at];
+      m = fmaxf(gates_s[at] + m, gates_s[plane + at]);
     }
-    __syncthreads();
-    if (threadIdx.x < heads) {
-      const int steps = count / heads;
-      int step = 0;
-      // Whole batches of eight tokens: sixteen loads, the chain in registers, twenty-four stores.
-      for (; step + 8 <= steps; step += 8) {
-        const int at0 = step * heads + threadIdx.x;
-        float f[8], i[8], a[8], b[8], c[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          f[u] = f_in[at0 + u * heads];
-          i[u] = i_in[at0 + u * heads];
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const float m_new = fmaxf(f[u] + m, i[u]);
-          a[u] = f[u] + m - m_new;
-          b[u] = i[u] - m_new;
-          c[u] = -m_new;
-          m = m_new;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          keep_o[at0 + u * heads] = a[u];
-          take_o[at0 + u * heads] = b[u];
-          floor_o[at0 + u * heads] = c[u];
-        }
-      }
-      for (int at = step * heads + threadIdx.x; at < count; at += heads) {
-        const float f = f_in[at], i = i_in[at];
-        const float m_new = fmaxf(f + m, i);
-        keep_o[at] = f + m - m_new;
-        take_o[at] = i - m_new;
-        floor_o[at] = -m_new;
-        m = m_new;
-      }
-    }
-    __syncthreads();
-    if (quads) {
-#pragma unroll 4
-      for (int idx = threadIdx.x * 4; idx < count; idx += blockDim.x * 4) {
-        *reinterpret_cast<float4*>(keep + base + idx) = *reinterpret_cast<const float4*>(keep_o + idx);
-        *reinterpret_cast<float4*>(take + base + idx) = *reinterpret_cast<const float4*>(take_o + idx);
-        *reinterpret_cast<float4*>(floor_out + base + idx) = *reinterpret_cast<const float4*>(floor_o + idx);
-      }
-    } else {
-      for (int idx = threadIdx.x; idx < count; idx += blockDim.x) {
-        keep[base + idx] = keep_o[idx];
-        take[base + idx] = take_o[idx];
-        floor_out[base + idx] = floor_o[idx];
-      }
-    }
-    __syncthreads();
+    a.moves_of(row, first, blockIdx.x)[h] = make_float2(sum, m);
+    if (blockIdx.x == 0) a.before[(size_t)row * a.heads + h] = a.state[(size_t)a.seq_seat[row] * a.heads + h];
   }
-  if (slot) *slot = m;
 }
 
-__global__ void exp_three_kernel(float* __restrict__ a, float* __restrict__ b, float* __restrict__ c, size_t total) {
-  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
-    a[idx] = expf(a[idx]);
-    b[idx] = expf(b[idx]);
-    c[idx] = expf(c[idx]);
+// Dynamic shared memory: 3 * chunk * heads floats.
+__global__ void __launch_bounds__(kGateThreads) exp_gate_walk_kernel(GateScan a) {
+  extern __shared__ float gates_s[];
+  const int row = blockIdx.y, first = a.seq_bounds[row], t0 = first + blockIdx.x * a.chunk, end = a.seq_bounds[row + 1];
+  if (t0 >= end) return;
+  const int count = min(a.chunk, end - t0) * a.heads, plane = a.chunk * a.heads;
+  const size_t base = (size_t)t0 * a.heads;
+  for (int idx = threadIdx.x; idx < count; idx += kGateThreads) {
+    gates_s[idx] = a.keep[base + idx];
+    gates_s[plane + idx] = a.take[base + idx];
+  }
+  __syncthreads();
+  for (int h = threadIdx.x; h < a.heads; h += kGateThreads) {
+    float m = a.before[(size_t)row * a.heads + h];
+    const float2* moves = a.moves_of(row, first, 0) + h;
+#pragma unroll 8
+    for (int c = 0; c < (int)blockIdx.x; ++c) {
+      const float2 move = moves[(size_t)c * a.heads];
+      m = fmaxf(move.x + m, move.y);
+    }
+    for (int at = h; at < count; at += a.heads) {
+      const float f = gates_s[at], i = gates_s[plane + at], m_new = fmaxf(f + m, i);
+      gates_s[at] = f + m - m_new;
+      gates_s[plane + at] = i - m_new;
+      gates_s[2 * plane + at] = -m_new;
+      m = m_new;
+    }
+    if (t0 + a.chunk >= end) a.state[(size_t)a.seq_seat[row] * a.heads + h] = m;
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < count; idx += kGateThreads) {
+    a.keep[base + idx] = expf(gates_s[idx]);
+    a.take[base + idx] = expf(gates_s[plane + idx]);
+    a.floor_out[base + idx] = expf(gates_s[2 * plane + idx]);
   }
 }
 
@@ -1213,32 +1198,36 @@ extern "C" int distie_activation(const float* x, int x_stride, int splits, long 
 
 // log_in and log_forget [tokens, heads] (views of one projection: the same slices); keep, take, floor [tokens, heads]
 // contiguous; state [seats, heads].
+// Floats of scratch that distie_exp_gate_scan takes.
+extern "C" long long distie_exp_gate_scratch_floats(int num_seqs, int tokens, int heads) {
+  if (heads < 1 || heads > 512) return 0;
+  return (2LL * (tokens / gate_chunk(heads) + num_seqs + 1) + num_seqs) * heads;
+}
+
+// scratch: 8-byte aligned; not read in a step of single tokens (tokens == num_seqs).
 extern "C" int distie_exp_gate_scan(const float* log_in, const float* log_forget, int gate_stride, int splits,
                                     long long split_stride, const float* in_bias, const float* forget_bias, float cap,
                                     float* state, const int* seq_bounds, const int* seq_seat, int num_seqs, int tokens,
-                                    int heads, float* keep, float* take, float* floor_out, cudaStream_t stream) {
+                                    int heads, float* keep, float* take, float* floor_out, float* scratch, cudaStream_t stream) {
   if (num_seqs <= 0) return 0;
   if (heads < 1 || splits < 1 || !(cap > 0.f) || state == nullptr || in_bias == nullptr || forget_bias == nullptr)
     return DISTIE_ERR_ARG;
-  if (heads > 512 || tokens < 1) return DISTIE_ERR_UNSUPPORTED;
-  const size_t total = (size_t)tokens * heads;
-  const unsigned blocks = (unsigned)((total + 255) / 256 > 148 * 8 ? 148 * 8 : (total + 255) / 256);
-  exp_gates_kernel<<<blocks, 256, 0, stream>>>(Sliced{log_in, gate_stride, splits, split_stride},
-                                              Sliced{log_forget, gate_stride, splits, split_stride}, in_bias, forget_bias,
-                                              cap, tokens, heads, keep, take);
+  if (heads > 512 || tokens < 1 || num_seqs > 65535) return DISTIE_ERR_UNSUPPORTED;
+  GateScan a{Sliced{log_in, gate_stride, splits, split_stride}, Sliced{log_forget, gate_stride, splits, split_stride}, in_bias,
+             forget_bias, cap, state, seq_bounds, seq_seat, heads, gate_chunk(heads), keep, take, floor_out, nullptr, nullptr};
+  if (tokens == num_seqs) {
+    exp_gate_single_kernel<<<(num_seqs * heads + kGateThreads - 1) / kGateThreads, kGateThreads, 0, stream>>>(a, num_seqs);
+    DISTIE_LAUNCH_CHECK();
+    return 0;
+  }
+  if (scratch == nullptr || ((uintptr_t)scratch & 7)) return DISTIE_ERR_ARG;
+  a.moves = reinterpret_cast<float2*>(scratch);
+  a.before = scratch + 2LL * (tokens / a.chunk + num_seqs + 1) * heads;
+  const dim3 grid((tokens + a.chunk - 1) / a.chunk, num_seqs);
+  const size_t plane = (size_t)a.chunk * heads * sizeof(float);  // at most 16 KB
+  exp_gate_moves_kernel<<<grid, kGateThreads, 2 * plane, stream>>>(a);
   DISTIE_LAUNCH_CHECK();
-  // Tiles as long as 160 KB of shared memory allow (512 tokens up to 16 heads): a tile costs a round trip to memory
-  // on either side of its walk, which only a long tile makes small beside the walk.
-  int tile_tokens = 8192 / (heads < 16 ? 16 : heads);
-  if (tile_tokens < 1) tile_tokens = 1;
-  if (tile_tokens > tokens) tile_tokens = tokens;
-  const size_t scan_shared = 5 * (size_t)tile_tokens * heads * sizeof(float);
-  if (scan_shared > 48 * 1024)
-    cudaFuncSetAttribute(exp_gate_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_shared);
-  exp_gate_scan_kernel<<<num_seqs, 512, scan_shared, stream>>>(
-      state, seq_bounds, seq_seat, heads, tile_tokens, keep, take, floor_out);
-  DISTIE_LAUNCH_CHECK();
-  exp_three_kernel<<<blocks, 256, 0, stream>>>(keep, take, floor_out, total);
+  exp_gate_walk_kernel<<<grid, kGateThreads, 3 * plane, stream>>>(a);
   DISTIE_LAUNCH_CHECK();
   return 0;
 }

@@ -975,15 +975,21 @@ class DeviceKernels(KernelSet):
             raise KernelError("exp_gate_scan: the two gates are views of one projection")
         heads = log_in.shape[-1]
         gates = torch.empty((3, step.num_tokens, heads), dtype=torch.float32, device=self.device)
+        single = step.num_tokens == step.num_seqs
+        scratch = None
+        if not single:
+            floats = function("distie_exp_gate_scratch_floats")(step.num_seqs, step.num_tokens, heads)
+            scratch = torch.empty(floats, dtype=torch.float32, device=self.device)
         check(
             function("distie_exp_gate_scan")(
                 in_ptr, forget_ptr, stride, splits, split_stride, in_bias.data_ptr(), forget_bias.data_ptr(), float(cap),
                 state.data_ptr(), self._seq_index(step)[1].data_ptr(), step.seq_seat.data_ptr(), step.num_seqs,
-                step.num_tokens, heads, gates[0].data_ptr(), gates[1].data_ptr(), gates[2].data_ptr(), self._stream(),
+                step.num_tokens, heads, gates[0].data_ptr(), gates[1].data_ptr(), gates[2].data_ptr(),
+                scratch.data_ptr() if scratch is not None else None, self._stream(),
             ),
             "exp_gate_scan",
         )
-        self._ran("exp_gate_scan", 3)
+        self._ran("exp_gate_scan", 1 if single else 2)
         return gates[0], gates[1], gates[2]
 
     def stabilized_readout(self, read, floor, heads, value_dim):

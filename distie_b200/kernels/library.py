@@ -89,7 +89,8 @@ _SIGNATURES: dict[str, tuple[str, list]] = {
     "distie_selective_scan_scratch_floats": ("channel", [I, I, I]),
     "distie_channel_delta": ("channel", [P, I, I, L, P, I, I, L, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P, P]),
     "distie_channel_delta_scratch_floats": ("channel", [I, I, I]),
-    "distie_exp_gate_scan": ("state", [P, P, I, I, L, P, P, F, P, P, P, I, I, I, P, P, P, P]),
+    "distie_exp_gate_scratch_floats": ("state", [I, I, I]),
+    "distie_exp_gate_scan": ("state", [P, P, I, I, L, P, P, F, P, P, P, I, I, I, P, P, P, P, P]),
     "distie_stabilized_readout": ("state", [P, I, P, P, I, I, I, P]),
     "distie_route_top": ("routed", [P, I, P, I, I, I, I, P, P, I, I, F, I, P, I, P, I, P, I, P]),
     "distie_route_pick": ("routed", [P, I, I, I, I, P, P, I, I, F, I, P, I, P, P]),
@@ -126,7 +127,8 @@ _SIGNATURES: dict[str, tuple[str, list]] = {
     "distie_gemm_tcgen05_skinny_act": ("bf16", [P, I, P, P, I, I, I, I, I, F, F, I, P, P]),
     "distie_gemm_tcgen05_skinny": ("bf16", [P, I, P, P, P, I, I, I, I, I, I, I, P, P]),
 }
-_RESULT = {"distie_retention_scratch_floats": c_longlong, "distie_recurrence_chunks_scratch_floats": c_longlong, "distie_attention_decode_scratch_floats": c_longlong, "distie_route_plan_words": c_longlong,
+_RESULT = {"distie_retention_scratch_floats": c_longlong, "distie_recurrence_chunks_scratch_floats": c_longlong,
+           "distie_exp_gate_scratch_floats": c_longlong, "distie_attention_decode_scratch_floats": c_longlong, "distie_route_plan_words": c_longlong,
            "distie_latent_attention_scratch_floats": c_longlong, "distie_selective_scan_scratch_floats": c_longlong,
            "distie_channel_delta_scratch_floats": c_longlong}
 

@@ -53,7 +53,9 @@ struct ChunkArgs {
   const int *q_tiles, *token_seq, *seq_seat;
   int tiles, heads, groups, key_dim, value_dim, v_dim;
   int* error;
-};
+  float q_scale;      // gated rule: q is multiplied by it
+  const float* floor; // gated rule with a unit column, [tokens, heads], or null.  Given: what leaves are the v_dim read-outs of
+};                    // a head divided by max(|the unit column's|, floor) + 1e-6, without the unit column's own
 
 constexpr int kRuleDelta = 0, kRuleSsd = 1, kRuleGated = 2;
 
@@ -269,6 +271,10 @@ struct Rows {
       x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (c < padded) x[i] = *reinterpret_cast<const float4*>(src + ((size_t)(c >> 4) * kChunk + row(i)) * 16 + (c & 15));
     }
+  }
+  __device__ __forceinline__ void scale(float s) {
+#pragma unroll
+    for (int i = 0; i < kMine; ++i) x[i] = make_float4(x[i].x * s, x[i].y * s, x[i].z * s, x[i].w * s);
   }
   // Rows of at most 128 elements made unit vectors, times `scale`.
   __device__ __forceinline__ void make_unit(float scale) {
@@ -811,6 +817,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a
       fetched_q.make_unit(rsqrtf((float)a.key_dim));
       fetched_k.make_unit(1.f);
     }
+    if (RULE == kRuleGated) fetched_q.scale(a.q_scale);
     fetched_q.store(q, kChunk, rows, a.key_dim, key_padded, nullptr, false);
     fetched_k.store(k, kChunk, rows, a.key_dim, key_padded, nullptr, false);
     fetched_S.store(S, value_padded, a.value_dim, a.key_dim, key_padded, nullptr, false);
@@ -870,8 +877,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a
   __syncthreads();
 
   const float skip = (RULE == kRuleSsd && a.skip) ? a.skip[head] : 0.f;
-  float* out = a.out + (size_t)t0 * a.out_stride + (size_t)head * a.value_dim;
-  const bool pairs = (a.value_dim & 1) == 0 && (a.out_stride & 1) == 0 && ((uintptr_t)a.out & 7) == 0;
+  const bool divided = RULE == kRuleGated && a.floor;
+  const int columns = divided ? a.v_dim : a.value_dim;
+  float* out = a.out + (size_t)t0 * a.out_stride + (size_t)head * columns;
+  const bool pairs = (columns & 1) == 0 && (a.out_stride & 1) == 0 && ((uintptr_t)a.out & 7) == 0;
   const auto p_at = first_rows(p, rg * 16, lane);
 #pragma unroll
   for (int i = 0; i < kUnits; ++i) {
@@ -888,20 +897,43 @@ __global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a
 #pragma unroll
     for (int n = 0; n < 2; ++n)
 #pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        o[i][n][r] += acc.of(n, r);
+        if (divided && unit * 16 + 8 * n + 2 * c + (r & 1) == a.v_dim) d.g[row0 + 8 * (r >> 1)] = o[i][n][r];  // (the g are done with)
+      }
+  }
+  float over[2] = {1.f, 1.f};
+  if (divided) {
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (row0 + 8 * h < rows)
+        over[h] = fmaxf(fabsf(d.g[row0 + 8 * h]), a.floor[(size_t)(t0 + row0 + 8 * h) * a.heads + head]) + 1e-6f;
+  }
+#pragma unroll
+  for (int i = 0; i < kUnits; ++i) {
+    const int unit = cq + 4 * i;
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int row = row0 + 8 * h, col = unit * 16 + 8 * n + 2 * c;
-        if (row >= rows || col >= a.value_dim) continue;
-        float x = o[i][n][2 * h] + acc.of(n, 2 * h), y = o[i][n][2 * h + 1] + acc.of(n, 2 * h + 1);
+        if (unit >= units || row >= rows || col >= columns) continue;
+        float x = o[i][n][2 * h], y = o[i][n][2 * h + 1];
         if (RULE == kRuleSsd) {
           const float* v = v_rows + (size_t)row * a.v_stride + col;
           x += skip * v[0];
-          if (col + 1 < a.value_dim) y += skip * v[1];
+          if (col + 1 < columns) y += skip * v[1];
+        }
+        if (divided) {
+          x /= over[h];
+          y /= over[h];
         }
         float* to = out + (size_t)row * a.out_stride + col;
         if (pairs) *reinterpret_cast<float2*>(to) = make_float2(x, y);
         else {
           to[0] = x;
-          if (col + 1 < a.value_dim) to[1] = y;
+          if (col + 1 < columns) to[1] = y;
         }
       }
   }
@@ -919,18 +951,19 @@ extern "C" long long distie_recurrence_chunks_scratch_floats(int rule, int tiles
 
 // The tokens of `q_tiles` ([tiles, 2] int32: first token, rows <= 128; the tiles of a request follow one another) under a
 // rule of distie_linear_recurrence, whose arguments these are, except that q and k stay as they are.  scratch: 16-byte
-// aligned.  -2: sizes that the kernels do not take (key_dim up to 128, value_dim up to 144).
+// aligned.  q_scale and floor: gated rule (see ChunkArgs; floor null and q_scale 1 otherwise; with a floor `out` holds the
+// divided read-outs, heads * (value_dim - 1) columns).  -2: sizes that the kernels do not take (key_dim up to 128, value_dim up to 144).
 extern "C" int distie_recurrence_chunks(int rule, const float* q, int q_stride, const float* k, int k_stride, const float* v,
                                         int v_stride, const float* decay, int decay_stride, const float* write, int write_stride,
                                         int splits, long long split_stride, const float* rate, const float* bias, const float* skip,
                                         float* state, float* out, int out_stride, float* scratch, const int* q_tiles, int tiles,
                                         const int* token_seq, const int* seq_seat, int heads, int groups, int key_dim, int value_dim,
-                                        int unit_column, int* error, cudaStream_t stream) {
+                                        int unit_column, float q_scale, const float* floor, int* error, cudaStream_t stream) {
   if (tiles <= 0) return 0;
   if (!error || heads < 1 || groups < 1 || heads % groups || key_dim < 1 || value_dim < 1 || splits < 1 || !q_tiles || !scratch || !state ||
       rule < kRuleDelta || rule > kRuleGated || (rule == kRuleDelta && !decay) ||
       (rule != kRuleGated && (!rate || !write || unit_column)) || (rule == kRuleGated && !rate && !decay) ||
-      (unit_column && value_dim < 2))
+      (unit_column && value_dim < 2) || (floor && !unit_column))
     return DISTIE_ERR_ARG;
   if (key_dim > 128 || value_dim > 144 || tiles > 32767 || heads > 65535) return DISTIE_ERR_UNSUPPORTED;
   if ((uintptr_t)scratch & 15) return DISTIE_ERR_ARG;
@@ -950,6 +983,8 @@ extern "C" int distie_recurrence_chunks(int rule, const float* q, int q_stride, 
   a.tiles = tiles; a.heads = heads; a.groups = groups; a.key_dim = key_dim; a.value_dim = value_dim;
   a.v_dim = unit_column ? value_dim - 1 : value_dim;
   a.error = error;
+  a.q_scale = q_scale;
+  a.floor = floor;
   const dim3 grid(heads, 2 * tiles);
   const bool narrow = value_dim <= 128;
   auto launch = [&](auto kernel, dim3 blocks, int threads, size_t shared) -> int {

@@ -683,7 +683,7 @@ class DeviceKernels(KernelSet):
                 function("distie_recurrence_chunks")(
                     *head, chunks.data_ptr(), step.q_tiles.data_ptr(), step.num_q_tiles, step.token_seq.data_ptr(),
                     step.seq_seat.data_ptr(), heads, groups, key_dim, value_dim, int(bool(unit_column)),
-                    self.error_flag.data_ptr(), self._stream(),
+                    1.0, None, self.error_flag.data_ptr(), self._stream(),
                 ),
                 "recurrence_chunks",
             )
@@ -699,6 +699,32 @@ class DeviceKernels(KernelSet):
                 "linear_recurrence",
             )
             self._ran("linear_recurrence", 2)
+        return out
+
+    def stabilized_memory(self, qkv, q_scale, keep, take, floor, state, step, heads, key_dim, value_dim):
+        """A step of nothing but portions that run in chunks: the kernels read the projection as it is, scale q on the way
+        in and divide the read-out on the way out.  Everything else: the ops after one another."""
+        rows = qkv[0] if qkv.dim() == 3 and qkv.shape[0] == 1 else qkv
+        if step.num_decode_tokens or rows.dim() != 2 or not self._in_chunks("gated", state, step, heads, key_dim, value_dim + 1):
+            return super().stabilized_memory(qkv, q_scale, keep, take, floor, state, step, heads, key_dim, value_dim)
+        self._rows32(rows, "stabilized_memory")
+        if not (keep.is_contiguous() and take.is_contiguous() and floor.is_contiguous()):
+            raise KernelError("stabilized_memory: contiguous gates are expected")
+        columns, base = heads * key_dim, rows.data_ptr()
+        out = torch.empty((step.num_tokens, heads * value_dim), dtype=torch.float32, device=rows.device)
+        floats = function("distie_recurrence_chunks_scratch_floats")(_RULES["gated"], step.num_q_tiles, heads, key_dim, value_dim + 1)
+        chunks = torch.empty(floats, dtype=torch.float32, device=rows.device)
+        check(
+            function("distie_recurrence_chunks")(
+                _RULES["gated"], base, rows.stride(0), base + 4 * columns, rows.stride(0), base + 8 * columns, rows.stride(0),
+                keep.data_ptr(), heads, take.data_ptr(), heads, 1, 0, None, None, None, state.data_ptr(), out.data_ptr(),
+                out.stride(0), chunks.data_ptr(), step.q_tiles.data_ptr(), step.num_q_tiles, step.token_seq.data_ptr(),
+                step.seq_seat.data_ptr(), heads, heads, key_dim, value_dim + 1, 1, float(q_scale), floor.data_ptr(),
+                self.error_flag.data_ptr(), self._stream(),
+            ),
+            "recurrence_chunks",
+        )
+        self._ran("recurrence_chunks", 3)
         return out
 
     def _in_chunks(self, rule, state, step, heads, key_dim, value_dim) -> bool:

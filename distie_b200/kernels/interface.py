@@ -291,6 +291,18 @@ class KernelSet(ABC):
         ``max(|n . q|, floor[t, h]) + 1e-6``."""
         raise NotImplementedError
 
+    def stabilized_memory(self, qkv, q_scale: float, keep, take, floor, state, step: StepTensors, heads: int, key_dim: int,
+                          value_dim: int):
+        """A memory with exponential gates from its projection to the stabilised read-out: ``qkv`` float32 ``[T, heads *
+        (2 key_dim + value_dim)]`` (or slices) holds ``[q | k | v]``, q to be multiplied by ``q_scale``; ``keep, take, floor``
+        are what :meth:`exp_gate_scan` returns; ``state [seats, heads, value_dim + 1, key_dim]`` as
+        :meth:`linear_recurrence` takes it with a unit column.  Returns what :meth:`stabilized_readout` makes of that."""
+        columns = heads * key_dim
+        rows = self.activation(qkv, "none", scale=q_scale, scaled_columns=columns)
+        read = self.linear_recurrence("gated", rows[:, :columns], rows[:, columns : 2 * columns], rows[:, 2 * columns :], keep, take,
+                                      state, step, heads, heads, key_dim, value_dim + 1, unit_column=True)
+        return self.stabilized_readout(read, floor, heads, value_dim)
+
     def route_top(self, x, router, top: int, scoring: str = "sigmoid", groups: tuple[int, int] | None = None,
                   weight_scale: float = 1.0, extra_rows: int = 0, correction=None, normalise: bool = False,
                   logit_bias=None):

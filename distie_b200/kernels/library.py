@@ -72,7 +72,7 @@ _SIGNATURES: dict[str, tuple[str, list]] = {
     ),
     "distie_recurrence_chunks_scratch_floats": ("state", [I, I, I, I, I]),
     "distie_recurrence_chunks": (
-        "state", [I, P, I, P, I, P, I, P, I, P, I, I, L, P, P, P, P, P, I, P, P, I, P, P, I, I, I, I, I, P, P]
+        "state", [I, P, I, P, I, P, I, P, I, P, I, I, L, P, P, P, P, P, I, P, P, I, P, P, I, I, I, I, I, F, P, P, P]
     ),
     "distie_activation": ("state", [P, I, I, L, P, I, I, I, F, I, I, P]),
     "distie_retention_scratch_floats": ("state", [I, I, I, I]),

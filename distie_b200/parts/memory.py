@@ -176,13 +176,10 @@ class ExpGateMemory:
         heads, qk, vv = self.heads, self.heads * self.key_dim, self.heads * self.value_dim
         y = k.linear_split(x, self.proj.weight)
         at = 2 * qk + vv
-        qkv = k.activation(y[:, :, :at], "none", scale=self.key_dim ** -0.5, scaled_columns=qk)
         keep, take, floor = k.exp_gate_scan(y[:, :, at : at + heads], y[:, :, at + heads : at + 2 * heads],
                                             self.vectors["i.b"], self.vectors["f.b"], self.cap, run.state["max"], run.step)
-        read = k.linear_recurrence("gated", qkv[:, :qk], qkv[:, qk : 2 * qk], qkv[:, 2 * qk :], keep, take,
-                                   run.state["matrix"], run.step, heads, heads, self.key_dim, self.value_dim + 1,
-                                   unit_column=True)
-        plain = k.stabilized_readout(read, floor, heads, self.value_dim)
+        plain = k.stabilized_memory(y[:, :, :at], self.key_dim ** -0.5, keep, take, floor, run.state["matrix"], run.step, heads,
+                                    self.key_dim, self.value_dim)
         normed = torch.empty((x.shape[0], vv), dtype=x.dtype, device=x.device)
         k.gated_rmsnorm(plain, y[:, :, at + 2 * heads :], self.vectors["norm"], self.eps, self.value_dim, False, normed,
                         activation="sigmoid")

@@ -610,7 +610,9 @@ template <int BN, int STAGES, int KB, int EPI>
 __global__ void __launch_bounds__(kGemmWideThreads, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          void* __restrict__ out, int ldo, int M, int N, int K, int inter, int m_tiles, int num_tiles,
-                         const QkvEpilogue qkv, int* __restrict__ error) {
+                         int n_tiles, int split_blocks, const QkvEpilogue qkv, int* __restrict__ error) {
+  // The reduction may be split (float32 epilogue): behind the n_tiles columns of tiles of the first split_blocks stages of K
+  // come those of the next ones, whose sums go to the next slice [M, ldo] of the output.
   extern __shared__ unsigned char raw[];
   auto& sm = *reinterpret_cast<PairShared<BN, STAGES, KB>*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
   constexpr uint32_t TMEM_COLS = 512;   // two accumulators, the second at column 256
@@ -622,6 +624,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const int k_blocks = (K + STAGE_K - 1) / STAGE_K;
   const uint32_t rank = cluster_cta_rank();       // 0: issues the MMAs
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  auto split_of = [&](int tile) { return EPI == GEMM_EPI_F32 ? tile / m_tiles / n_tiles : 0; };
+  auto column_of = [&](int tile) { return (tile / m_tiles - split_of(tile) * n_tiles) * PER_TILE; };
+  auto blocks_of = [&](int tile) { return min(split_blocks, k_blocks - split_of(tile) * split_blocks); };
 
   if (threadIdx.x == 64) {
     prefetch_tensor_map(&map_a);
@@ -657,25 +662,25 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       bool ok = true;
       // Rows of W this CTA stages: with SwiGLU the first CTA takes the gate rows, the second the up rows.
       auto rows_of_w = [&](int tile) {
-        const int n_tile = (tile / m_tiles) * PER_TILE;
+        const int n_tile = column_of(tile);
         return EPI == GEMM_EPI_SWIGLU ? (rank == 0 ? n_tile : inter + n_tile) : n_tile + (int)rank * (BN / 2);
       };
       // The weights are written by no kernel: the first ring of them is on its way before the wait for
       // the kernel that makes the activations.  (A copy of the second CTA may land on the first CTA's
       // barrier before that one has announced the bytes; the phase cannot end before it has.)
-      const int early = pair < num_tiles ? min(k_blocks, STAGES) : 0;
+      const int early = pair < num_tiles ? min(blocks_of(pair), STAGES) : 0;
       for (int kb = 0; kb < early; ++kb) {
         if (rank == 0) mbar_expect_tx(&sm.full[kb], STAGE_BYTES_PAIR);
         const uint32_t full_addr = cluster_address(&sm.full[kb], 0);
 #pragma unroll
         for (int box = 0; box < KB; ++box)
-          tma_load_2d_pair(sm.b[kb][box], &map_b, full_addr, kb * STAGE_K + box * kGemmBK, rows_of_w(pair));
+          tma_load_2d_pair(sm.b[kb][box], &map_b, full_addr, (split_of(pair) * split_blocks + kb) * STAGE_K + box * kGemmBK, rows_of_w(pair));
       }
       grid_dependency_wait();
       for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
         const int m0 = (tile % m_tiles) * 2 * kGemmBM + (int)rank * kGemmBM;
-        const int w0 = rows_of_w(tile);
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        const int w0 = rows_of_w(tile), k0 = split_of(tile) * split_blocks * STAGE_K, tile_blocks = blocks_of(tile);
+        for (int kb = 0; kb < tile_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           const bool ahead = it < (uint32_t)early;  // this stage's weights are under way already
           if (!ahead) {
@@ -685,8 +690,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           const uint32_t full_addr = cluster_address(&sm.full[s], 0);
 #pragma unroll
           for (int box = 0; box < KB; ++box) {  // a box past K is filled with zeros and still counted
-            tma_load_2d_pair(sm.a[s][box], &map_a, full_addr, kb * STAGE_K + box * kGemmBK, m0);
-            if (!ahead) tma_load_2d_pair(sm.b[s][box], &map_b, full_addr, kb * STAGE_K + box * kGemmBK, w0);
+            tma_load_2d_pair(sm.a[s][box], &map_a, full_addr, k0 + kb * STAGE_K + box * kGemmBK, m0);
+            if (!ahead) tma_load_2d_pair(sm.b[s][box], &map_b, full_addr, k0 + kb * STAGE_K + box * kGemmBK, w0);
           }
         }
       }
@@ -710,7 +715,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         if (!mbar_wait_unless(&sm.accum_empty[buffer], ((round >> 1) & 1) ^ 1, &sm.failed)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem + buffer * ACC_STRIDE;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        const int tile_blocks = blocks_of(tile);
+        for (int kb = 0; kb < tile_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait_unless(&sm.full[s], (it / STAGES) & 1, &sm.failed)) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -738,7 +744,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     for (int tile = pair; tile < num_tiles; tile += pairs, ++round) {
       const uint32_t buffer = round & 1;
       const int m0 = (tile % m_tiles) * 2 * kGemmBM + (int)rank * kGemmBM;
-      const int n0 = (tile / m_tiles) * PER_TILE;
+      const int n0 = column_of(tile);
       if (EPI == GEMM_EPI_QKV) {  // this warp's cos and sin, on their way while the tile's MMAs run
         if (qkv.head_dim == 128) qkv_stage_trig<128>(trig_stage, m0 + quadrant * 32, lane, part, M, qkv.trig);
         else qkv_stage_trig<64>(trig_stage, m0 + quadrant * 32, lane, part, M, qkv.trig);
@@ -751,7 +757,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         if (qkv.head_dim == 128) store_qkv_rope<128>(lane_base, m0 + quadrant * 32, lane, n0, part, (__nv_bfloat16*)out, ldo, M, N, qkv, trig_stage);
         else store_qkv_rope<64>(lane_base, m0 + quadrant * 32, lane, n0, part, (__nv_bfloat16*)out, ldo, M, N, qkv, trig_stage);
       } else {
-        store_accumulator<BN, EPI>(lane_base, m0 + quadrant * 32, lane, n0, out, ldo, M, N, inter, part, epilogue_stage,
+        void* slice = EPI == GEMM_EPI_F32 ? static_cast<void*>(static_cast<float*>(out) + (size_t)split_of(tile) * M * ldo) : out;
+        store_accumulator<BN, EPI>(lane_base, m0 + quadrant * 32, lane, n0, slice, ldo, M, N, inter, part, epilogue_stage,
                                    qkv.act.a, qkv.act);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -997,7 +1004,8 @@ static int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, void*
 
 template <int BN, int STAGES, int KB, int EPI>
 static int launch_gemm_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, void* out, int ldo, int M, int N, int K,
-                            int inter, int sm_count, int* error, cudaStream_t stream, const QkvEpilogue& qkv = QkvEpilogue()) {
+                            int inter, int sm_count, int* error, cudaStream_t stream, const QkvEpilogue& qkv = QkvEpilogue(),
+                            int splits = 1) {
   const size_t shared = sizeof(PairShared<BN, STAGES, KB>) + 1024 + (EPI == GEMM_EPI_QKV ? 16 + 8 * kQkvStageFloats * sizeof(float) : 0) +
                         (EPI == GEMM_EPI_F32 ? 16 + 8 * kEpilogueStageBytes : 0);
   static bool configured = false;
@@ -1025,12 +1033,15 @@ static int launch_gemm_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, 
   const int m_tiles = (M + 2 * kGemmBM - 1) / (2 * kGemmBM);
   const int columns = EPI == GEMM_EPI_SWIGLU ? inter : N;
   const int per_tile = EPI == GEMM_EPI_SWIGLU ? BN / 2 : BN;
-  const int num_tiles = m_tiles * ((columns + per_tile - 1) / per_tile);
+  const int n_tiles = (columns + per_tile - 1) / per_tile, k_blocks = (K + KB * kGemmBK - 1) / (KB * kGemmBK);
+  const int split_blocks = (k_blocks + splits - 1) / splits;
+  if ((k_blocks + split_blocks - 1) / split_blocks != splits) return DISTIE_ERR_ARG;  // (no slice without a share of K)
+  const int num_tiles = m_tiles * n_tiles * splits;
   const int slots = resident_pairs < sm_count / 2 ? resident_pairs : sm_count / 2;
   const int pairs = num_tiles < slots ? num_tiles : slots;
   const cudaError_t err = launch_dependent_cluster(64, dim3(2, 1, 1), gemm_tcgen05_pair_kernel<BN, STAGES, KB, EPI>,
                                                    dim3(2 * pairs), dim3(kGemmWideThreads), shared, stream, map_a, map_b, out,
-                                                   ldo, M, N, K, inter, m_tiles, num_tiles, qkv, error);
+                                                   ldo, M, N, K, inter, m_tiles, num_tiles, n_tiles, split_blocks, qkv, error);
   return err == cudaSuccess ? 0 : (int)err;
 }
 
@@ -1138,6 +1149,32 @@ extern "C" int distie_gemm_tcgen05_act(const void* x, int ldx, const void* w, vo
   if (width == 192) { DISTIE_GEMM(192, 5, 4); }
   DISTIE_GEMM(128, 6, 6);
 #undef DISTIE_GEMM
+}
+
+// The slices of a product of few columns: at 256 rows and more, its tiles of 256 x 128 would leave most of the machine idle
+// while a few pairs of CTAs walk the whole of K.  `splits` pairs share a tile's K (as many stages of 64 each but for the last
+// one) and leave slices [splits, M, N] float32 whose sum is the product, for consumers that add slices up.
+// distie_gemm_tcgen05_splits: how many slices that is; 1: not worth it (a quarter of the pairs are busy already, or a share
+// would be shorter than four stages).  1,024 x 128 x 3,072: 28 -> 8 us with 8 slices.
+extern "C" int distie_gemm_tcgen05_splits(int M, int N, int K, int sm_count) {
+  if (M < 2 * kGemmBM || N < 1 || K < 1 || sm_count < 2) return 1;
+  const int tiles = (M + 2 * kGemmBM - 1) / (2 * kGemmBM) * ((N + 127) / 128), k_blocks = (K + kGemmBK - 1) / kGemmBK;
+  int splits = min(8, min(sm_count / 2 / tiles, k_blocks / 4));
+  if (tiles > sm_count / 8 || splits < 2) return 1;
+  const int share = (k_blocks + splits - 1) / splits;
+  return (k_blocks + share - 1) / share;
+}
+extern "C" int distie_gemm_tcgen05_split(const void* x, int ldx, const void* w, float* out, int M, int N, int K, int splits,
+                                         int sm_count, int* error, cudaStream_t stream) {
+  if (M <= 0) return 0;
+  if (M < 2 * kGemmBM || N < 1 || K < 8 || splits < 1 || (K & 7) || (ldx & 7) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15))
+    return DISTIE_ERR_UNSUPPORTED;
+  if (sm_count < 2) sm_count = 148;
+  CUtensorMap map_a, map_b;
+  int status = make_map(&map_a, x, M, K, ldx, kGemmBM);
+  if (status == 0) status = make_map(&map_b, w, N, K, K, 64);
+  if (status != 0) return status;
+  return launch_gemm_pair<128, 8, 1, GEMM_EPI_F32>(map_a, map_b, out, N, M, N, K, 0, sm_count, error, stream, QkvEpilogue(), splits);
 }
 
 // The grouped product (see gemm_tcgen05_grouped_kernel): a[rows_a, K] sorted by group, w[groups * w_rows, K]; the tile

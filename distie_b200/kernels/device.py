@@ -144,7 +144,25 @@ class DeviceKernels(KernelSet):
             out = torch.empty((splits, m, n), dtype=torch.float32, device=x.device)
             self._stream_weights(x, weight, None, out, 0)
             return out
+        if self._tensor_core(x, weight):
+            m, n, k = x.shape[0], weight.shape[0], weight.shape[1]
+            splits = function("distie_gemm_tcgen05_splits")(m, n, k, self.sm_count)
+            if splits > 1:
+                return self._gemm_split(x, weight, splits)
         return super().linear_split(x, weight)
+
+    def _gemm_split(self, x, weight, splits: int):
+        out = torch.empty((splits, x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
+        check(
+            function("distie_gemm_tcgen05_split")(
+                x.data_ptr(), x.stride(0), weight.data_ptr(), out.data_ptr(), x.shape[0], weight.shape[0], weight.shape[1],
+                splits, self.sm_count, self.error_flag.data_ptr(), self._stream(),
+            ),
+            "gemm_tcgen05_split",
+        )
+        self._ran("gemm_tcgen05")
+        self._ran("gemm_tcgen05_split", 0)
+        return out
 
     def linear(self, x, weight, bias=None, out_dtype=None):
         out_dtype = out_dtype or self.dtype
@@ -1053,14 +1071,18 @@ class DeviceKernels(KernelSet):
         if self._tensor_core(x, router):
             # Prompt portions in bfloat16: the logits are a product on the tcgen05 tile kernel (float32 accumulators,
             # stored as float32), and a small kernel picks from them.
-            logits = torch.empty((tokens, experts + extra), dtype=torch.float32, device=x.device)
-            self._gemm_tcgen05(x, router, logits, 1)
-            check(function("distie_route_pick")(logits.data_ptr(), logits.stride(0), tokens, experts, top, ids.data_ptr(),
-                                                weights.data_ptr(), count, keep, float(weight_scale), softmax, correction_ptr,
-                                                norm, bias_ptr, self._stream()),
+            splits = 1 if extra else function("distie_gemm_tcgen05_splits")(tokens, experts, x.shape[1], self.sm_count)
+            if splits > 1:  # (few columns: the slices of its split reduction are added up as they are read)
+                logits = self._gemm_split(x, router, splits)
+            else:
+                logits = torch.empty((1, tokens, experts + extra), dtype=torch.float32, device=x.device)
+                self._gemm_tcgen05(x, router, logits[0], 1)
+            check(function("distie_route_pick")(logits.data_ptr(), logits.stride(1), splits, logits.stride(0), tokens, experts, top,
+                                                ids.data_ptr(), weights.data_ptr(), count, keep, float(weight_scale), softmax,
+                                                correction_ptr, norm, bias_ptr, self._stream()),
                   "route_pick")
             self._ran("route_top")
-            return (ids, weights, logits[:, experts:]) if extra else (ids, weights)
+            return (ids, weights, logits[0, :, experts:]) if extra else (ids, weights)
         extra_out = torch.empty((tokens, extra), dtype=torch.float32, device=x.device) if extra else None
         check(
             function("distie_route_top")(x.data_ptr(), x.stride(0), router.data_ptr(), tokens, x.shape[1], experts, top,

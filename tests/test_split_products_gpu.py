@@ -1,0 +1,42 @@
+"""Products of few columns whose reduction is split over pairs of CTAs, against the product in 64 bits.
+
+The operands are bfloat16 and the sums float32: K additions of 2^-24 each in a chain are at most sqrt(K) * 2^-23 of the
+result's norm, and truncating accumulators K / 16 * 2^-24 more."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k", [(256, 1, 512), (257, 16, 1536), (1001, 128, 3080), (2048, 130, 1000), (640, 250, 4096), (511, 96, 584)])
+def test_slices_add_up_to_the_product(m, n, k):
+    from distie_b200.kernels import make_kernels
+
+    ks = make_kernels(torch.bfloat16, "cuda:0")
+    generator = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(m, k, generator=generator, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(n, k, generator=generator, device="cuda") / k**0.5).to(torch.bfloat16)
+    slices = ks.linear_split(x, w)
+    ks.check_errors()
+    assert "gemm_tcgen05_split" in ks.kernel_counts and slices.shape[0] > 1 and slices.shape[1:] == (m, n)
+    want = x.double() @ w.double().t()
+    error = float((slices.double().sum(0) - want).norm() / want.norm())
+    assert error <= k**0.5 * 2**-23 + k / 16 * 2**-24, f"off by {error:.2e}"
+
+
+def test_the_router_reads_the_slices():
+    from distie_b200.kernels import make_kernels
+
+    ks = make_kernels(torch.bfloat16, "cuda:0")
+    generator = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(700, 1536, generator=generator, device="cuda").to(torch.bfloat16)
+    router = (torch.randn(24, 1536, generator=generator, device="cuda") / 40).to(torch.bfloat16)
+    ids, weights = ks.route_top(x, router, 3)
+    score = torch.sigmoid(x.double() @ router.double().t())
+    top, want = score.topk(4, -1)
+    clear = (top[:, :3] - top[:, 1:] > 1e-5).all(-1)
+    assert int(clear.sum()) > 650 and torch.equal(ids[clear].long(), want[clear, :3])
+    assert float((weights.double() - top[:, :3])[clear].abs().max()) < 1e-5

@@ -144,7 +144,7 @@ class DeviceKernels(KernelSet):
             out = torch.empty((splits, m, n), dtype=torch.float32, device=x.device)
             self._stream_weights(x, weight, None, out, 0)
             return out
-        if self._tensor_core(x, weight):
+        if self._tensor_core(x, weight) and not self._underfilled(x, weight):
             m, n, k = x.shape[0], weight.shape[0], weight.shape[1]
             splits = function("distie_gemm_tcgen05_splits")(m, n, k, self.sm_count)
             if splits > 1:

@@ -26,6 +26,11 @@
 //
 // Why chunks: the walk is a chain of about 110 dependent instructions a token and head column, 0.15 to 0.25 us a token
 // whatever the machine could do beside it.  Single tokens and short portions stay on it (the rule is in kernels/device.py).
+// 2,048 tokens of 12 heads of 128: 372 us in the walk, 92 in chunks (state-space duality); 507 and 169 (delta rule).
+//
+// What bounds the kernels: mma.sync (1,024 multiply-adds a cycle and SM; 12 for a 16 x 16 x 16 step) and the reads of shared
+// memory that feed it, each about a third of a block's time, behind loads that a block makes once and the splitting of
+// operands into parts; chunk_walk the chain itself, 2.4 us a chunk.
 #include "recurrent.cuh"
 #include "tcgen05.cuh"
 
@@ -649,7 +654,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(ChunkArgs a
   float S[4];
   const size_t size = (size_t)a.value_dim * a.key_dim;
   float* slot = a.state + ((size_t)a.seq_seat[seq] * a.heads + head) * size;
-  const bool pairs = (a.key_dim & 1) == 0;
+  const bool pairs = (a.key_dim & 1) == 0 && ((uintptr_t)a.state & 7) == 0;
   const int col0 = warp * 8 + 2 * c, row0 = slice * 16 + g;
 #pragma unroll
   for (int r = 0; r < 4; ++r) {

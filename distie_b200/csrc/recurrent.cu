@@ -807,7 +807,7 @@ struct GateScan {
   float cap;
   float* state;
   const int *seq_bounds, *seq_seat;
-  int heads, chunk;
+  int heads, chunk, row0;  // row0: the request of blockIdx.y == 0
   float *keep, *take, *floor_out;
   float2* moves;  // [tokens / chunk + requests + 1, heads]: F and I
   float* before;  // [requests, heads]: m before the step
@@ -837,7 +837,7 @@ __global__ void __launch_bounds__(kGateThreads) exp_gate_single_kernel(GateScan 
 // Dynamic shared memory: 2 * chunk * heads floats.
 __global__ void __launch_bounds__(kGateThreads) exp_gate_moves_kernel(GateScan a) {
   extern __shared__ float gates_s[];
-  const int row = blockIdx.y, first = a.seq_bounds[row], t0 = first + blockIdx.x * a.chunk, end = a.seq_bounds[row + 1];
+  const int row = a.row0 + blockIdx.y, first = a.seq_bounds[row], t0 = first + blockIdx.x * a.chunk, end = a.seq_bounds[row + 1];
   if (t0 >= end) return;
   const int count = min(a.chunk, end - t0) * a.heads, plane = a.chunk * a.heads;
   for (int idx = threadIdx.x; idx < count; idx += kGateThreads) {
@@ -864,7 +864,7 @@ __global__ void __launch_bounds__(kGateThreads) exp_gate_moves_kernel(GateScan a
 // Dynamic shared memory: 3 * chunk * heads floats.
 __global__ void __launch_bounds__(kGateThreads) exp_gate_walk_kernel(GateScan a) {
   extern __shared__ float gates_s[];
-  const int row = blockIdx.y, first = a.seq_bounds[row], t0 = first + blockIdx.x * a.chunk, end = a.seq_bounds[row + 1];
+  const int row = a.row0 + blockIdx.y, first = a.seq_bounds[row], t0 = first + blockIdx.x * a.chunk, end = a.seq_bounds[row + 1];
   if (t0 >= end) return;
   const int count = min(a.chunk, end - t0) * a.heads, plane = a.chunk * a.heads;
   const size_t base = (size_t)t0 * a.heads;
@@ -1212,9 +1212,9 @@ extern "C" int distie_exp_gate_scan(const float* log_in, const float* log_forget
   if (num_seqs <= 0) return 0;
   if (heads < 1 || splits < 1 || !(cap > 0.f) || state == nullptr || in_bias == nullptr || forget_bias == nullptr)
     return DISTIE_ERR_ARG;
-  if (heads > 512 || tokens < 1 || num_seqs > 65535) return DISTIE_ERR_UNSUPPORTED;
+  if (heads > 512 || tokens < 1) return DISTIE_ERR_UNSUPPORTED;
   GateScan a{Sliced{log_in, gate_stride, splits, split_stride}, Sliced{log_forget, gate_stride, splits, split_stride}, in_bias,
-             forget_bias, cap, state, seq_bounds, seq_seat, heads, gate_chunk(heads), keep, take, floor_out, nullptr, nullptr};
+             forget_bias, cap, state, seq_bounds, seq_seat, heads, gate_chunk(heads), 0, keep, take, floor_out, nullptr, nullptr};
   if (tokens == num_seqs) {
     exp_gate_single_kernel<<<(num_seqs * heads + kGateThreads - 1) / kGateThreads, kGateThreads, 0, stream>>>(a, num_seqs);
     DISTIE_LAUNCH_CHECK();
@@ -1223,12 +1223,15 @@ extern "C" int distie_exp_gate_scan(const float* log_in, const float* log_forget
   if (scratch == nullptr || ((uintptr_t)scratch & 7)) return DISTIE_ERR_ARG;
   a.moves = reinterpret_cast<float2*>(scratch);
   a.before = scratch + 2LL * (tokens / a.chunk + num_seqs + 1) * heads;
-  const dim3 grid((tokens + a.chunk - 1) / a.chunk, num_seqs);
   const size_t plane = (size_t)a.chunk * heads * sizeof(float);  // at most 16 KB
-  exp_gate_moves_kernel<<<grid, kGateThreads, 2 * plane, stream>>>(a);
-  DISTIE_LAUNCH_CHECK();
-  exp_gate_walk_kernel<<<grid, kGateThreads, 3 * plane, stream>>>(a);
-  DISTIE_LAUNCH_CHECK();
+  constexpr int kRowsAtOnce = 65535;
+  for (a.row0 = 0; a.row0 < num_seqs; a.row0 += kRowsAtOnce) {
+    const dim3 grid((tokens + a.chunk - 1) / a.chunk, num_seqs - a.row0 < kRowsAtOnce ? num_seqs - a.row0 : kRowsAtOnce);
+    exp_gate_moves_kernel<<<grid, kGateThreads, 2 * plane, stream>>>(a);
+    DISTIE_LAUNCH_CHECK();
+    exp_gate_walk_kernel<<<grid, kGateThreads, 3 * plane, stream>>>(a);
+    DISTIE_LAUNCH_CHECK();
+  }
   return 0;
 }
 

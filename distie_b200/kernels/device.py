@@ -761,7 +761,7 @@ class DeviceKernels(KernelSet):
         portions, rest = step.num_seqs - singles, step.num_tokens - singles
         return (self.dtype == torch.bfloat16 and portions > 0 and step.num_q_tiles > 0
                 and rest >= _CHUNKS_FROM[rule][0] * portions + _CHUNKS_FROM[rule][1] / heads
-                and key_dim <= 128 and value_dim <= 144 and state.is_contiguous()
+                and key_dim <= 128 and value_dim <= 144 and step.num_q_tiles <= 32767 and state.is_contiguous()
                 and 4 * function("distie_recurrence_chunks_scratch_floats")(_RULES[rule], step.num_q_tiles, heads, key_dim,
                                                                             value_dim) <= _CHUNK_BYTES)
 

@@ -224,7 +224,7 @@ route_top_kernel(const T* __restrict__ x, int x_stride, const T* __restrict__ ro
 
 // The choice alone, from float32 logits [tokens, experts] that a product left: a warp per token.
 __global__ void __launch_bounds__(kRouteThreads)
-route_pick_kernel(const float* __restrict__ logits, int logit_stride, int splits, long long split_stride, int tokens, int experts, int top,
+route_pick_kernel(const float* __restrict__ logits, int logit_stride, int tokens, int experts, int top,
                   int* __restrict__ ids, float* __restrict__ weights, int group_count, int group_keep, float weight_scale,
                   int softmax, const float* __restrict__ correction, int normalise, const float* __restrict__ logit_bias) {
   extern __shared__ float pick_s[];  // per warp: a row of scores, group_count floats, a row of plain scores
@@ -233,9 +233,7 @@ route_pick_kernel(const float* __restrict__ logits, int logit_stride, int splits
   if (t >= tokens) return;
   float* mine = pick_s + (size_t)warp * (2 * experts + group_count);
   for (int e = lane; e < experts; e += 32) {
-    float z = logits[(size_t)t * logit_stride + e];
-    for (int s = 1; s < splits; ++s) z += logits[(size_t)s * split_stride + (size_t)t * logit_stride + e];
-    if (logit_bias) z += logit_bias[e];
+    const float z = logits[(size_t)t * logit_stride + e] + (logit_bias ? logit_bias[e] : 0.f);
     mine[e] = softmax ? z : routed_sigmoid(z);
   }
   __syncwarp();
@@ -921,20 +919,19 @@ extern "C" int distie_routed_scatter(const float* y, int* plan, int pairs, int e
   return 0;
 }
 
-// ids and weights from float32 logits [tokens, experts] (row stride logit_stride; or `splits` slices of a split product,
-// split_stride floats apart, which are added up): see route_pick_kernel.
-extern "C" int distie_route_pick(const float* logits, int logit_stride, int splits, long long split_stride, int tokens, int experts, int top, int* ids,
+// ids and weights from float32 logits [tokens, experts] (row stride logit_stride): see route_pick_kernel.
+extern "C" int distie_route_pick(const float* logits, int logit_stride, int tokens, int experts, int top, int* ids,
                                  float* weights, int group_count, int group_keep, float weight_scale, int softmax,
                                  const float* correction, int normalise, const float* logit_bias, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (correction != nullptr && group_count > 1 && group_keep < group_count) return DISTIE_ERR_ARG;
-  if (splits < 1 || experts < 1 || top < 1 || top > experts || top > kMaxTop || experts > 4096 || group_count < 1 ||
+  if (experts < 1 || top < 1 || top > experts || top > kMaxTop || experts > 4096 || group_count < 1 ||
       experts % group_count != 0 || group_keep < 1 || group_keep > group_count || top > group_keep * (experts / group_count))
     return DISTIE_ERR_ARG;
   const int warps = kRouteThreads / 32;
   const size_t shared = (size_t)warps * (2 * experts + group_count) * sizeof(float);
   if (shared > 48 * 1024) cudaFuncSetAttribute(route_pick_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-  route_pick_kernel<<<(tokens + warps - 1) / warps, kRouteThreads, shared, stream>>>(logits, logit_stride, splits, split_stride, tokens, experts,
+  route_pick_kernel<<<(tokens + warps - 1) / warps, kRouteThreads, shared, stream>>>(logits, logit_stride, tokens, experts,
                                                                                     top, ids, weights, group_count, group_keep,
                                                                                     weight_scale, softmax, correction, normalise,
                                                                                     logit_bias);

@@ -1080,18 +1080,15 @@ class DeviceKernels(KernelSet):
         if self._tensor_core(x, router):
             # Prompt portions in bfloat16: the logits are a product on the tcgen05 tile kernel (float32 accumulators,
             # stored as float32), and a small kernel picks from them.
-            splits = 1 if extra else function("distie_gemm_tcgen05_splits")(tokens, experts, x.shape[1], self.sm_count)
-            if splits > 1:  # (few columns: the slices of its split reduction are added up as they are read)
-                logits = self._gemm_split(x, router, splits)
-            else:
-                logits = torch.empty((1, tokens, experts + extra), dtype=torch.float32, device=x.device)
-                self._gemm_tcgen05(x, router, logits[0], 1)
-            check(function("distie_route_pick")(logits.data_ptr(), logits.stride(1), splits, logits.stride(0), tokens, experts, top,
-                                                ids.data_ptr(), weights.data_ptr(), count, keep, float(weight_scale), softmax,
-                                                correction_ptr, norm, bias_ptr, self._stream()),
+            # One whole product whatever the step's size: with a tie within rounding, other orders of summation choose other experts.
+            logits = torch.empty((tokens, experts + extra), dtype=torch.float32, device=x.device)
+            self._gemm_tcgen05(x, router, logits, 1)
+            check(function("distie_route_pick")(logits.data_ptr(), logits.stride(0), tokens, experts, top, ids.data_ptr(),
+                                                weights.data_ptr(), count, keep, float(weight_scale), softmax, correction_ptr,
+                                                norm, bias_ptr, self._stream()),
                   "route_pick")
             self._ran("route_top")
-            return (ids, weights, logits[0, :, experts:]) if extra else (ids, weights)
+            return (ids, weights, logits[:, experts:]) if extra else (ids, weights)
         extra_out = torch.empty((tokens, extra), dtype=torch.float32, device=x.device) if extra else None
         check(
             function("distie_route_top")(x.data_ptr(), x.stride(0), router.data_ptr(), tokens, x.shape[1], experts, top,

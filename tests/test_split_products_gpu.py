@@ -27,7 +27,7 @@ def test_slices_add_up_to_the_product(m, n, k):
     assert error <= k**0.5 * 2**-23 + k / 16 * 2**-24, f"off by {error:.2e}"
 
 
-def test_the_router_reads_the_slices():
+def test_the_router_against_the_product_in_64_bits():
     from distie_b200.kernels import make_kernels
 
     ks = make_kernels(torch.bfloat16, "cuda:0")
@@ -40,3 +40,19 @@ def test_the_router_reads_the_slices():
     clear = (top[:, :3] - top[:, 1:] > 1e-5).all(-1)
     assert int(clear.sum()) > 650 and torch.equal(ids[clear].long(), want[clear, :3])
     assert float((weights.double() - top[:, :3])[clear].abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("experts,width", [(16, 1536), (256, 1024), (64, 3584)])
+def test_a_token_is_routed_alike_in_every_step(experts, width):
+    """Chosen experts are whole numbers: a token's must not hang on how many tokens share its step.  (The logits are one
+    product in one order of summation from 256 rows on; 6,000 rows are more tiles than any split takes.)"""
+    from distie_b200.kernels import make_kernels
+
+    ks = make_kernels(torch.bfloat16, "cuda:0")
+    generator = torch.Generator(device="cuda").manual_seed(9)
+    x = torch.randn(6000, width, generator=generator, device="cuda").to(torch.bfloat16)
+    router = (torch.randn(experts, width, generator=generator, device="cuda") / width**0.5).to(torch.bfloat16)
+    ids, weights = ks.route_top(x, router, 3)
+    for rows in (300, 1001, 2048):
+        few_ids, few_weights = ks.route_top(x[:rows], router, 3)
+        assert torch.equal(few_ids, ids[:rows]) and torch.equal(few_weights, weights[:rows])

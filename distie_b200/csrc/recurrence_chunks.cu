@@ -25,7 +25,8 @@
 // (A value that is not finite spoils the whole chunk of its request, as it spoils all later tokens in the walk.)
 //
 // Why chunks: the walk is a chain of about 110 dependent instructions a token and head column, 0.15 to 0.25 us a token
-// whatever the machine could do beside it.  Single tokens and short portions stay on it (the rule is in kernels/device.py).
+// whatever the machine could do beside it.  Single tokens, short portions and many portions of small states, which fill the
+// machine, stay on it (chunks_pay in kernels/device.py).
 // 2,048 tokens of 12 heads of 128: 372 us in the walk, 92 in chunks (state-space duality); 507 and 169 (delta rule).
 //
 // What bounds the kernels: mma.sync (1,024 multiply-adds a cycle and SM; 12 for a 16 x 16 x 16 step) and the reads of shared

@@ -19,6 +19,7 @@ import numpy as np
 import torch
 
 import ctypes
+import math
 from dataclasses import replace
 
 from . import library
@@ -34,7 +35,6 @@ _CLUSTER_SPLITS = 8             # splits of a decode attention that one cluster 
 _TENSOR_CORE_ROWS = 128         # from here on the tcgen05 kernel's 128-row tiles are full; in between: the library
 _MAX_TERMS = 24                 # terms of a pending sum that the layer-norm kernel adds up itself
 _RULES = {"delta": 0, "ssd": 1, "gated": 2}
-_CHUNKS_FROM = {"delta": (110, 500), "ssd": (48, 1700), "gated": (48, 1700)}  # tokens a portion, and tokens times heads a step
 _CHUNK_BYTES = 1 << 30          # the most that the states between the chunks of a step may take
 _ACTS = {"relu2": 1, "gelu": 2, "xielu": 3}
 _SCORINGS = {"sigmoid": 0, "softmax": 1, "softmax_chosen": 2}
@@ -52,6 +52,34 @@ _ERROR_TEXT = {
     7: "a router chose an expert that does not exist",
     5: "a block table does not cover the keys a portion of a prompt attends to",
 }
+
+
+def chunks_pay(rule: str, tokens: int, portions: int, heads: int, key_dim: int, value_dim: int) -> bool:
+    """Whether ``portions`` portions of ``tokens`` tokens together are faster in chunks of 64 tokens (recurrence_chunks.cu)
+    than in the walk token by token (recurrent.cu).
+
+    Two estimates in us, fitted to 4,700 steps timed both ways (keys and values of 16 to 128, 1 to 64 heads, 1 to 32 portions
+    of 24 to 1,024 tokens; each within 10 % of the times).  The walk: a token of a portion costs the latency of its chain or, once the
+    columns fill the machine, its share of the arithmetic, which grows with the sizes.  The chunks: the blocks' latency, which
+    hardly shrinks with the sizes, then whole blocks of 64 tokens and a head.  So the chunks win on long portions of few heads
+    and on large states, and the walk on many short portions of small ones (walk / chunks, us; delta rule: one portion of 2,048
+    tokens of 12 heads of 128 507 / 169, sixteen of 155 of 40 heads of 16 66 / 248; state-space duality: 372 / 92, and sixteen
+    of 71 of 40 heads of 16 28 / 82).  A portion's length enters as the mean, at which the walk is never slower than it
+    would be with one portion longer than the others.  0.95, and 96 tokens for the delta rule: where the estimates err."""
+    mean = tokens / portions
+    wide, keys, values = (32 if key_dim <= 32 else 64 if key_dim <= 64 else 128), -(-key_dim // 16) / 8, -(-value_dim // 16) / 8
+    columns, blocks = portions * heads * value_dim, portions * -(-mean // 64) * heads
+    if rule == "delta":
+        if mean < 96:
+            return False
+        chain = (0.138 + 0.0526 * math.log2(wide / 32), (7.12 + 0.422 * wide) * columns * 1e-6)
+        walk = 8.1 + mean * (chain[0] ** 2.8 + chain[1] ** 2.8) ** (1 / 2.8) + 3.3e-4 * tokens * heads
+        chunks = 19.6 + 0.4 * mean / 64 + (4.8 + 2.8 * keys + 6.0 * values + 10.5 * keys * values) * max(1.0, blocks * 2.43 / 148)
+    else:
+        chain = (0.109 + 0.0195 * math.log2(wide / 32), (4.84 + 0.392 * wide) * columns * 1e-6)
+        walk = 6.5 + mean * math.hypot(*chain) + 1.8e-4 * tokens * heads
+        chunks = 9.1 + 0.23 * mean / 64 + (6.1 + 2.0 * values + 12.8 * keys * values) * max(1.0, blocks * 1.36 / 148 + 0.19)
+    return chunks < 0.95 * walk
 
 
 class DeviceKernels(KernelSet):
@@ -747,21 +775,12 @@ class DeviceKernels(KernelSet):
 
     def _in_chunks(self, rule, state, step, heads, key_dim, value_dim) -> bool:
         """Whether the portions of a step run in chunks of 64 tokens instead of token by token (16-bit engine: the
-        float32 engine's sums stay on the FMA pipe).
-
-        The walk takes 0.18 us a token of the longest portion while its columns do not fill the machine, and grows with
-        the tokens of the step once they do; the chunks cost about 30 us and then 0.05 us a token and 12 heads.  Measured
-        with heads of 128 (walk / chunks, us): one portion, 12 heads, 128 tokens 28 / 33, 192 tokens 40 / 34, 2,048
-        tokens 372 / 92; 28 heads, 96 tokens 31 / 34, 128 tokens 40 / 34; four portions of 64 with 12 heads 27 / 34, of
-        96 38 / 35; sixteen of 33 54 / 65, of 64 92 / 70.  The delta rule's chunks cost more (solving for the writes):
-        one portion, 12 heads, 128 tokens 38 / 41, 192 tokens 53 / 44, 2,048 tokens 507 / 169; 28 heads, 128 tokens
-        47 / 48; four portions of 128 with 12 heads 55 / 55; sixteen of 96 150 / 170, of 128 196 / 171.  The lines of
-        _CHUNKS_FROM lie between these."""
+        float32 engine's sums stay on the FMA pipe)."""
         singles = step.num_decode_tokens
         portions, rest = step.num_seqs - singles, step.num_tokens - singles
         return (self.dtype == torch.bfloat16 and portions > 0 and step.num_q_tiles > 0
-                and rest >= _CHUNKS_FROM[rule][0] * portions + _CHUNKS_FROM[rule][1] / heads
-                and key_dim <= 128 and value_dim <= 144 and step.num_q_tiles <= 32767 and state.is_contiguous()
+                and key_dim <= 128 and value_dim <= 144 and chunks_pay(rule, rest, portions, heads, key_dim, value_dim)
+                and step.num_q_tiles <= 32767 and state.is_contiguous()
                 and 4 * function("distie_recurrence_chunks_scratch_floats")(_RULES[rule], step.num_q_tiles, heads, key_dim,
                                                                             value_dim) <= _CHUNK_BYTES)
 

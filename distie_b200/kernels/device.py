@@ -82,6 +82,23 @@ def chunks_pay(rule: str, tokens: int, portions: int, heads: int, key_dim: int, 
     return chunks < 0.95 * walk
 
 
+def tiles_pay(tokens: int, portions: int, keys: int, heads: int, size: int) -> bool:
+    """Whether float32 attention of ``portions`` portions of ``tokens`` tokens together, that see up to ``keys`` keys, is
+    faster on tiles of 32 rows and 64 keys (attention_tiles.cu) than with a block per token and head (attention_generic.cu);
+    ``size``: the larger of a head's keys and values.
+
+    Two estimates in us, fitted to 12,000 steps timed both ways (heads of 16 to 128, 1 to 40 of them, 1 to 32 portions of 2 to
+    128 tokens behind up to 1,000): the one kernel pays for every key of a token, the other for whole tiles however few
+    of their rows are there.  So a few rows over a few keys are the first one's (us, without and with tiles: sixteen portions of 8
+    tokens, 40 heads of 128 14.6 / 34.2; sixteen of 2 behind 70 25.7 / 57.8; 8 rows alone 4.5 / 9.5, behind 1,000 keys
+    241 / 102; 500 rows 373 / 60).  0.9: where the estimates err."""
+    wide, mean = (32 if size <= 32 else 64 if size <= 64 else 128) / 128, tokens / portions
+    blocks = portions * -(-mean // 32) * heads
+    plain = 3.0 + (0.6 + 0.3 * size / 128) * -(-keys // 4) * max(1.0, tokens * heads / 710) ** 0.81 + 0.113 * tokens * heads / 148
+    tiled = 2.4 + (2.2 + 5.2 * wide) * -(-keys // 64) * max(1.0, blocks / 296) + 5.2 * wide * blocks / 148
+    return tiled < 0.9 * plain
+
+
 class DeviceKernels(KernelSet):
     def __init__(self, dtype: torch.dtype, device: torch.device | str = "cuda:0") -> None:
         if dtype not in _CODE:
@@ -544,14 +561,11 @@ class DeviceKernels(KernelSet):
 
     def _attention_tiles(self, qkv, out, step, kv, num_heads, num_kv_heads, head_dim, window, chunk, scale, keep_first,
                          softcap, sink_ptr) -> bool:
-        """Portions of the float32 engine on the tiled kernel; False when it refuses a size or an alignment.
-
-        A block of it takes 32 rows and keys 64 at a time, so a few rows over a few keys stay on the size-agnostic kernel:
-        that one takes 0.24 us a key of the longest row and the tiles 7 to 10 us and then 0.1 us a key (12 and 28 heads of
-        128; 8 rows alone: 4.5 against 9.5 us, behind 1,000 keys 241 against 102; 32 rows alone: 10.5 against 10.0;
-        500: 373 against 60)."""
-        rows = step.num_tokens - step.num_decode_tokens
-        if self.dtype != torch.float32 or not step.num_q_tiles or (rows < 32 and step.max_kv_len <= 64):
+        """Portions of the float32 engine on the tiled kernel; False where the size-agnostic one is faster, or when the
+        kernel refuses a size or an alignment."""
+        portions = step.num_seqs - step.num_decode_tokens
+        if self.dtype != torch.float32 or not step.num_q_tiles or portions < 1 or not tiles_pay(
+                step.num_tokens - step.num_decode_tokens, portions, step.max_kv_len, num_heads, max(head_dim, kv.v.shape[-1])):
             return False
         code = function("distie_attention_tiles")(
             qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), step.q_tiles.data_ptr(), step.num_q_tiles,

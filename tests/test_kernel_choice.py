@@ -7,7 +7,7 @@ from __future__ import annotations
 
 import pytest
 
-from distie_b200.kernels.device import chunks_pay
+from distie_b200.kernels.device import chunks_pay, tiles_pay
 
 
 @pytest.mark.parametrize("rule,key,value,heads,portions,tokens,walk,chunks", [
@@ -31,3 +31,20 @@ from distie_b200.kernels.device import chunks_pay
 ])
 def test_recurrences_run_in_chunks_where_that_is_faster(rule, key, value, heads, portions, tokens, walk, chunks):
     assert chunks_pay(rule, portions * tokens, portions, heads, key, value) == (chunks < walk)
+
+
+@pytest.mark.parametrize("heads,size,portions,tokens,past,plain,tiles", [
+    # heads, their size, portions, tokens of each, tokens before them, us with a block per token and head, us in tiles
+    (40, 128, 32, 2, 0, 7.3, 57.9),
+    (40, 128, 16, 8, 0, 14.6, 34.2),
+    (40, 128, 16, 2, 70, 25.7, 57.8),
+    (12, 128, 32, 2, 0, 4.5, 24.6),
+    (2, 64, 16, 8, 0, 3.9, 6.9),
+    (2, 16, 1, 128, 300, 72.7, 21.6),
+    (28, 16, 32, 6, 128, 146.7, 37.8),
+    (1, 32, 8, 4, 1000, 168.2, 45.7),
+    (40, 64, 8, 24, 1000, 1466.0, 120.3),
+    (12, 32, 8, 3, 300, 54.9, 27.1),
+])
+def test_float32_attention_runs_in_tiles_where_that_is_faster(heads, size, portions, tokens, past, plain, tiles):
+    assert tiles_pay(portions * tokens, portions, tokens + past, heads, size) == (tiles < plain)

@@ -799,7 +799,15 @@ __global__ void activation_kernel(Sliced x, T* __restrict__ out, int tokens, int
 // tokens of 12 heads, with 5 us around it; these two take 8.)
 // ---------------------------------------------------------------------------
 constexpr int kGateThreads = 256;
-__host__ __device__ constexpr int gate_chunk(int heads) { return heads <= 64 ? 64 : 4096 / heads; }  // tokens (512 heads: 8)
+// The tokens of a step's longest portion when every request has one at least (it sizes chunks and grids and bounds nothing).
+__host__ __device__ constexpr int max_portion(int num_seqs, int tokens) { return tokens > num_seqs ? tokens - num_seqs + 1 : 1; }
+// Tokens of a chunk.  Short portions: few, so that their gates are made by more than a block or two and no chain is long;
+// long ones: many, because every chunk folds those before it.  (One portion of 64 tokens, 12, 28 and 70 heads, us: chunks of
+// 64 10.0, 12.8, 17.8.)  At most 4,096 gates a block (512 heads: 8 tokens).
+__host__ __device__ constexpr int gate_chunk(int num_seqs, int tokens, int heads) {
+  const int longest = max_portion(num_seqs, tokens), wanted = longest <= 128 ? 8 : longest <= 512 ? 16 : longest <= 1024 ? 32 : 64;
+  return wanted * heads <= 4096 ? wanted : 4096 / heads;
+}
 
 struct GateScan {
   Sliced log_in, log_forget;
@@ -823,78 +831,95 @@ struct GateScan {
 __global__ void __launch_bounds__(kGateThreads) exp_gate_single_kernel(GateScan a, int rows) {
   const int idx = blockIdx.x * kGateThreads + threadIdx.x;
   if (idx >= rows * a.heads) return;
-  const int row = idx / a.heads, h = idx % a.heads, t = a.seq_bounds[row];
-  if (a.seq_bounds[row + 1] <= t) return;
+  const int row = idx / a.heads, h = idx % a.heads, end = a.seq_bounds[row + 1];
   float* slot = a.state + (size_t)a.seq_seat[row] * a.heads + h;
-  const float f = a.forget_gate(t, h), i = a.in_gate(t, h), m = *slot, m_new = fmaxf(f + m, i);
-  const size_t at = (size_t)t * a.heads + h;
-  a.keep[at] = expf(f + m - m_new);
-  a.take[at] = expf(i - m_new);
-  a.floor_out[at] = expf(-m_new);
-  *slot = m_new;
+  for (int t = a.seq_bounds[row]; t < end; ++t) {  // one
+    const float f = a.forget_gate(t, h), i = a.in_gate(t, h), m = *slot, m_new = fmaxf(f + m, i);
+    const size_t at = (size_t)t * a.heads + h;
+    a.keep[at] = expf(f + m - m_new);
+    a.take[at] = expf(i - m_new);
+    a.floor_out[at] = expf(-m_new);
+    *slot = m_new;
+  }
 }
 
 // Dynamic shared memory: 2 * chunk * heads floats.
 __global__ void __launch_bounds__(kGateThreads) exp_gate_moves_kernel(GateScan a) {
   extern __shared__ float gates_s[];
-  const int row = a.row0 + blockIdx.y, first = a.seq_bounds[row], t0 = first + blockIdx.x * a.chunk, end = a.seq_bounds[row + 1];
-  if (t0 >= end) return;
-  const int count = min(a.chunk, end - t0) * a.heads, plane = a.chunk * a.heads;
-  for (int idx = threadIdx.x; idx < count; idx += kGateThreads) {
-    const size_t t = t0 + idx / a.heads;
-    const int h = idx % a.heads;
-    const float f = a.forget_gate(t, h), i = a.in_gate(t, h);
-    gates_s[idx] = f;
-    gates_s[plane + idx] = i;
-    a.keep[(size_t)t0 * a.heads + idx] = f;
-    a.take[(size_t)t0 * a.heads + idx] = i;
-  }
-  __syncthreads();
-  for (int h = threadIdx.x; h < a.heads; h += kGateThreads) {
-    float sum = 0.f, m = -INFINITY;
-    for (int at = h; at < count; at += a.heads) {
-      sum += gates_s[at];
-      m = fmaxf(gates_s[at] + m, gates_s[plane + at]);
+  const int row = a.row0 + blockIdx.y, first = a.seq_bounds[row], end = a.seq_bounds[row + 1], plane = a.chunk * a.heads;
+  for (int index = blockIdx.x, t0 = first + index * a.chunk; t0 < end; index += gridDim.x, t0 = first + index * a.chunk) {
+    const int count = min(a.chunk, end - t0) * a.heads;
+    for (int idx = threadIdx.x; idx < count; idx += kGateThreads) {
+      const size_t t = t0 + idx / a.heads;
+      const int h = idx % a.heads;
+      const float f = a.forget_gate(t, h), i = a.in_gate(t, h);
+      gates_s[idx] = f;
+      gates_s[plane + idx] = i;
+      a.keep[(size_t)t0 * a.heads + idx] = f;
+      a.take[(size_t)t0 * a.heads + idx] = i;
     }
-    a.moves_of(row, first, blockIdx.x)[h] = make_float2(sum, m);
-    if (blockIdx.x == 0) a.before[(size_t)row * a.heads + h] = a.state[(size_t)a.seq_seat[row] * a.heads + h];
+    __syncthreads();
+    for (int h = threadIdx.x; h < a.heads; h += kGateThreads) {
+      float sum = 0.f, m = -INFINITY;
+#pragma unroll 8
+      for (int at = h; at < count; at += a.heads) {
+        sum += gates_s[at];
+        m = fmaxf(gates_s[at] + m, gates_s[plane + at]);
+      }
+      a.moves_of(row, first, index)[h] = make_float2(sum, m);
+      if (index == 0) a.before[(size_t)row * a.heads + h] = a.state[(size_t)a.seq_seat[row] * a.heads + h];
+    }
+    __syncthreads();  // the gates may be overwritten
   }
 }
 
 // Dynamic shared memory: 3 * chunk * heads floats.
 __global__ void __launch_bounds__(kGateThreads) exp_gate_walk_kernel(GateScan a) {
   extern __shared__ float gates_s[];
-  const int row = a.row0 + blockIdx.y, first = a.seq_bounds[row], t0 = first + blockIdx.x * a.chunk, end = a.seq_bounds[row + 1];
-  if (t0 >= end) return;
-  const int count = min(a.chunk, end - t0) * a.heads, plane = a.chunk * a.heads;
-  const size_t base = (size_t)t0 * a.heads;
-  for (int idx = threadIdx.x; idx < count; idx += kGateThreads) {
-    gates_s[idx] = a.keep[base + idx];
-    gates_s[plane + idx] = a.take[base + idx];
-  }
-  __syncthreads();
-  for (int h = threadIdx.x; h < a.heads; h += kGateThreads) {
-    float m = a.before[(size_t)row * a.heads + h];
-    const float2* moves = a.moves_of(row, first, 0) + h;
+  const int row = a.row0 + blockIdx.y, first = a.seq_bounds[row], end = a.seq_bounds[row + 1], plane = a.chunk * a.heads;
+  for (int index = blockIdx.x, t0 = first + index * a.chunk; t0 < end; index += gridDim.x, t0 = first + index * a.chunk) {
+    const int count = min(a.chunk, end - t0) * a.heads;
+    const size_t base = (size_t)t0 * a.heads;
+    for (int idx = threadIdx.x; idx < count; idx += kGateThreads) {
+      gates_s[idx] = a.keep[base + idx];
+      gates_s[plane + idx] = a.take[base + idx];
+    }
+    __syncthreads();
+    for (int h = threadIdx.x; h < a.heads; h += kGateThreads) {
+      float m = a.before[(size_t)row * a.heads + h];
+      const float2* moves = a.moves_of(row, first, 0) + h;
 #pragma unroll 8
-    for (int c = 0; c < (int)blockIdx.x; ++c) {
-      const float2 move = moves[(size_t)c * a.heads];
-      m = fmaxf(move.x + m, move.y);
+      for (int c = 0; c < index; ++c) {
+        const float2 move = moves[(size_t)c * a.heads];
+        m = fmaxf(move.x + m, move.y);
+      }
+      for (int at = h; at < count; at += 8 * a.heads) {  // eight tokens: their loads, the chain in registers, their stores
+        float f[8], i[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const bool live = at + u * a.heads < count;
+          f[u] = live ? gates_s[at + u * a.heads] : 0.f;
+          i[u] = live ? gates_s[plane + at + u * a.heads] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (at + u * a.heads >= count) break;
+          const float m_new = fmaxf(f[u] + m, i[u]);
+          gates_s[at + u * a.heads] = f[u] + m - m_new;
+          gates_s[plane + at + u * a.heads] = i[u] - m_new;
+          gates_s[2 * plane + at + u * a.heads] = -m_new;
+          m = m_new;
+        }
+      }
+      if (t0 + a.chunk >= end) a.state[(size_t)a.seq_seat[row] * a.heads + h] = m;
     }
-    for (int at = h; at < count; at += a.heads) {
-      const float f = gates_s[at], i = gates_s[plane + at], m_new = fmaxf(f + m, i);
-      gates_s[at] = f + m - m_new;
-      gates_s[plane + at] = i - m_new;
-      gates_s[2 * plane + at] = -m_new;
-      m = m_new;
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < count; idx += kGateThreads) {
+      a.keep[base + idx] = expf(gates_s[idx]);
+      a.take[base + idx] = expf(gates_s[plane + idx]);
+      a.floor_out[base + idx] = expf(gates_s[2 * plane + idx]);
     }
-    if (t0 + a.chunk >= end) a.state[(size_t)a.seq_seat[row] * a.heads + h] = m;
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < count; idx += kGateThreads) {
-    a.keep[base + idx] = expf(gates_s[idx]);
-    a.take[base + idx] = expf(gates_s[plane + idx]);
-    a.floor_out[base + idx] = expf(gates_s[2 * plane + idx]);
+    __syncthreads();  // the gates may be overwritten
   }
 }
 
@@ -1196,15 +1221,14 @@ extern "C" int distie_activation(const float* x, int x_stride, int splits, long 
   return 0;
 }
 
-// log_in and log_forget [tokens, heads] (views of one projection: the same slices); keep, take, floor [tokens, heads]
-// contiguous; state [seats, heads].
 // Floats of scratch that distie_exp_gate_scan takes.
 extern "C" long long distie_exp_gate_scratch_floats(int num_seqs, int tokens, int heads) {
-  if (heads < 1 || heads > 512) return 0;
-  return (2LL * (tokens / gate_chunk(heads) + num_seqs + 1) + num_seqs) * heads;
+  if (heads < 1 || heads > 512 || tokens < 1 || num_seqs < 1) return 0;
+  return (2LL * (tokens / gate_chunk(num_seqs, tokens, heads) + num_seqs + 1) + num_seqs) * heads;
 }
 
-// scratch: 8-byte aligned; not read in a step of single tokens (tokens == num_seqs).
+// log_in and log_forget [tokens, heads] (views of one projection: the same slices); keep, take, floor [tokens, heads]
+// contiguous; state [seats, heads].  scratch: 8-byte aligned; not read in a step of single tokens (tokens == num_seqs).
 extern "C" int distie_exp_gate_scan(const float* log_in, const float* log_forget, int gate_stride, int splits,
                                     long long split_stride, const float* in_bias, const float* forget_bias, float cap,
                                     float* state, const int* seq_bounds, const int* seq_seat, int num_seqs, int tokens,
@@ -1214,7 +1238,7 @@ extern "C" int distie_exp_gate_scan(const float* log_in, const float* log_forget
     return DISTIE_ERR_ARG;
   if (heads > 512 || tokens < 1) return DISTIE_ERR_UNSUPPORTED;
   GateScan a{Sliced{log_in, gate_stride, splits, split_stride}, Sliced{log_forget, gate_stride, splits, split_stride}, in_bias,
-             forget_bias, cap, state, seq_bounds, seq_seat, heads, gate_chunk(heads), 0, keep, take, floor_out, nullptr, nullptr};
+             forget_bias, cap, state, seq_bounds, seq_seat, heads, gate_chunk(num_seqs, tokens, heads), 0, keep, take, floor_out, nullptr, nullptr};
   if (tokens == num_seqs) {
     exp_gate_single_kernel<<<(num_seqs * heads + kGateThreads - 1) / kGateThreads, kGateThreads, 0, stream>>>(a, num_seqs);
     DISTIE_LAUNCH_CHECK();
@@ -1226,7 +1250,7 @@ extern "C" int distie_exp_gate_scan(const float* log_in, const float* log_forget
   const size_t plane = (size_t)a.chunk * heads * sizeof(float);  // at most 16 KB
   constexpr int kRowsAtOnce = 65535;
   for (a.row0 = 0; a.row0 < num_seqs; a.row0 += kRowsAtOnce) {
-    const dim3 grid((tokens + a.chunk - 1) / a.chunk, num_seqs - a.row0 < kRowsAtOnce ? num_seqs - a.row0 : kRowsAtOnce);
+    const dim3 grid((max_portion(num_seqs, tokens) + a.chunk - 1) / a.chunk, num_seqs - a.row0 < kRowsAtOnce ? num_seqs - a.row0 : kRowsAtOnce);
     exp_gate_moves_kernel<<<grid, kGateThreads, 2 * plane, stream>>>(a);
     DISTIE_LAUNCH_CHECK();
     exp_gate_walk_kernel<<<grid, kGateThreads, 3 * plane, stream>>>(a);

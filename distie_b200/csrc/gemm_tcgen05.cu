@@ -606,13 +606,15 @@ struct PairShared {
   uint32_t failed;
 };
 
-template <int BN, int STAGES, int KB, int EPI>
+template <int BN, int STAGES, int KB, int EPI, bool SPLIT>
 __global__ void __launch_bounds__(kGemmWideThreads, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          void* __restrict__ out, int ldo, int M, int N, int K, int inter, int m_tiles, int num_tiles,
                          int n_tiles, int split_blocks, const QkvEpilogue qkv, int* __restrict__ error) {
-  // The reduction may be split (float32 epilogue): behind the n_tiles columns of tiles of the first split_blocks stages of K
-  // come those of the next ones, whose sums go to the next slice [M, ldo] of the output.
+  // SPLIT (float32 epilogue): behind the n_tiles columns of tiles of the first split_blocks stages of K come those of the next
+  // ones, whose sums go to the next slice [M, ldo] of the output.  A template: the divisions that find a tile's slice cost
+  // whole products 1.2 us a launch.
+  static_assert(!SPLIT || EPI == GEMM_EPI_F32, "slices are float32");
   extern __shared__ unsigned char raw[];
   auto& sm = *reinterpret_cast<PairShared<BN, STAGES, KB>*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
   constexpr uint32_t TMEM_COLS = 512;   // two accumulators, the second at column 256
@@ -624,9 +626,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const int k_blocks = (K + STAGE_K - 1) / STAGE_K;
   const uint32_t rank = cluster_cta_rank();       // 0: issues the MMAs
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  auto split_of = [&](int tile) { return EPI == GEMM_EPI_F32 ? tile / m_tiles / n_tiles : 0; };
+  auto split_of = [&](int tile) { return SPLIT ? tile / m_tiles / n_tiles : 0; };
   auto column_of = [&](int tile) { return (tile / m_tiles - split_of(tile) * n_tiles) * PER_TILE; };
-  auto blocks_of = [&](int tile) { return min(split_blocks, k_blocks - split_of(tile) * split_blocks); };
+  auto blocks_of = [&](int tile) { return SPLIT ? min(split_blocks, k_blocks - split_of(tile) * split_blocks) : k_blocks; };
 
   if (threadIdx.x == 64) {
     prefetch_tensor_map(&map_a);
@@ -757,7 +759,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         if (qkv.head_dim == 128) store_qkv_rope<128>(lane_base, m0 + quadrant * 32, lane, n0, part, (__nv_bfloat16*)out, ldo, M, N, qkv, trig_stage);
         else store_qkv_rope<64>(lane_base, m0 + quadrant * 32, lane, n0, part, (__nv_bfloat16*)out, ldo, M, N, qkv, trig_stage);
       } else {
-        void* slice = EPI == GEMM_EPI_F32 ? static_cast<void*>(static_cast<float*>(out) + (size_t)split_of(tile) * M * ldo) : out;
+        void* slice = SPLIT ? static_cast<void*>(static_cast<float*>(out) + (size_t)split_of(tile) * M * ldo) : out;
         store_accumulator<BN, EPI>(lane_base, m0 + quadrant * 32, lane, n0, slice, ldo, M, N, inter, part, epilogue_stage,
                                    qkv.act.a, qkv.act);
       }
@@ -1002,7 +1004,7 @@ static int launch_gemm(const CUtensorMap& map_a, const CUtensorMap& map_b, void*
   return err == cudaSuccess ? 0 : (int)err;
 }
 
-template <int BN, int STAGES, int KB, int EPI>
+template <int BN, int STAGES, int KB, int EPI, bool SPLIT = false>
 static int launch_gemm_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, void* out, int ldo, int M, int N, int K,
                             int inter, int sm_count, int* error, cudaStream_t stream, const QkvEpilogue& qkv = QkvEpilogue(),
                             int splits = 1) {
@@ -1011,7 +1013,7 @@ static int launch_gemm_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, 
   static bool configured = false;
   static int resident_pairs = 0;  // pairs that can run at the same time (an SM left over in a GPC hosts none)
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<BN, STAGES, KB, EPI>,
+    cudaError_t err = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<BN, STAGES, KB, EPI, SPLIT>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
     if (err != cudaSuccess) return (int)err;
     cudaLaunchConfig_t probe = {};
@@ -1025,7 +1027,7 @@ static int launch_gemm_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, 
     attribute[0].val.clusterDim.z = 1;
     probe.attrs = attribute;
     probe.numAttrs = 1;
-    err = cudaOccupancyMaxActiveClusters(&resident_pairs, gemm_tcgen05_pair_kernel<BN, STAGES, KB, EPI>, &probe);
+    err = cudaOccupancyMaxActiveClusters(&resident_pairs, gemm_tcgen05_pair_kernel<BN, STAGES, KB, EPI, SPLIT>, &probe);
     if (err != cudaSuccess) return (int)err;
     if (resident_pairs < 1) return DISTIE_ERR_UNSUPPORTED;
     configured = true;
@@ -1039,7 +1041,7 @@ static int launch_gemm_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, 
   const int num_tiles = m_tiles * n_tiles * splits;
   const int slots = resident_pairs < sm_count / 2 ? resident_pairs : sm_count / 2;
   const int pairs = num_tiles < slots ? num_tiles : slots;
-  const cudaError_t err = launch_dependent_cluster(64, dim3(2, 1, 1), gemm_tcgen05_pair_kernel<BN, STAGES, KB, EPI>,
+  const cudaError_t err = launch_dependent_cluster(64, dim3(2, 1, 1), gemm_tcgen05_pair_kernel<BN, STAGES, KB, EPI, SPLIT>,
                                                    dim3(2 * pairs), dim3(kGemmWideThreads), shared, stream, map_a, map_b, out,
                                                    ldo, M, N, K, inter, m_tiles, num_tiles, n_tiles, split_blocks, qkv, error);
   return err == cudaSuccess ? 0 : (int)err;
@@ -1176,7 +1178,8 @@ extern "C" int distie_gemm_tcgen05_split(const void* x, int ldx, const void* w, 
   int status = make_map(&map_a, x, M, K, ldx, kGemmBM);
   if (status == 0) status = make_map(&map_b, w, N, K, K, 64);
   if (status != 0) return status;
-  return launch_gemm_pair<128, 8, 1, GEMM_EPI_F32>(map_a, map_b, out, N, M, N, K, 0, sm_count, error, stream, QkvEpilogue(), splits);
+  return splits > 1 ? launch_gemm_pair<128, 8, 1, GEMM_EPI_F32, true>(map_a, map_b, out, N, M, N, K, 0, sm_count, error, stream, QkvEpilogue(), splits)
+                    : launch_gemm_pair<128, 8, 1, GEMM_EPI_F32>(map_a, map_b, out, N, M, N, K, 0, sm_count, error, stream);
 }
 
 // The grouped product (see gemm_tcgen05_grouped_kernel): a[rows_a, K] sorted by group, w[groups * w_rows, K]; the tile

@@ -889,14 +889,12 @@ class DeviceKernels(KernelSet):
     def selective_scan(self, x, dt, B, C, gate, rates, skip, dt_bias, state, step, out) -> None:
         self._rows32(x, "selective_scan x")
         states = rates.shape[0]
-        if B.dim() == 3 and B.shape[0] > 1 and step.num_decode_tokens < step.num_tokens:
-            # Every block of channels reads all of B and C: slices are added up once (1,024 tokens, 8 slices: 3 us here
-            # against 34 us in the scan).
-            if C.data_ptr() - B.data_ptr() == 4 * states and B.stride() == C.stride():
-                both = self.activation(B.as_strided((*B.shape[:2], 2 * states), B.stride()), "none")
-                B, C = both[:, :states], both[:, states:]
-            else:
-                B, C = self.activation(torch.cat([B, C], -1), "none").split(states, -1)
+        if (B.dim() == 3 and B.shape[0] > 1 and step.num_decode_tokens < step.num_tokens
+                and C.data_ptr() - B.data_ptr() == 4 * states and (B.shape, B.stride(), B.dtype) == (C.shape, C.stride(), C.dtype)):
+            # Every block of channels reads all of B and C: neighbours in the slices of one projection are added up once
+            # (1,024 tokens, 8 slices: 3 us here against 34 us in the scan).
+            both = self.activation(B.as_strided((*B.shape[:2], 2 * states), B.stride()), "none")
+            B, C = both[:, :states], both[:, states:]
         b_at, c_at = self._sliced(B, "selective_scan B"), self._sliced(C, "selective_scan C")
         if b_at[1:] != c_at[1:]:
             raise KernelError("selective_scan: B and C are views of one projection")

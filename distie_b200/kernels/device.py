@@ -889,10 +889,13 @@ class DeviceKernels(KernelSet):
     def selective_scan(self, x, dt, B, C, gate, rates, skip, dt_bias, state, step, out) -> None:
         self._rows32(x, "selective_scan x")
         states = rates.shape[0]
-        if (B.dim() == 3 and B.shape[0] > 1 and step.num_decode_tokens < step.num_tokens
+        rest, portions = step.num_tokens - step.num_decode_tokens, step.num_seqs - step.num_decode_tokens
+        if (B.dim() == 3 and B.shape[0] > 1 and rest > 0 and rest * states >= 512 * portions
                 and C.data_ptr() - B.data_ptr() == 4 * states and (B.shape, B.stride(), B.dtype) == (C.shape, C.stride(), C.dtype)):
             # Every block of channels reads all of B and C: neighbours in the slices of one projection are added up once
-            # (1,024 tokens, 8 slices: 3 us here against 34 us in the scan).
+            # (1,024 tokens, 8 slices: 3 us here against 34 us in the scan).  Portions of few tokens read the slices
+            # themselves, a launch less: layer without projections, added up here / in the scan, us, 3,072 channels of 16 states:
+            # eight portions of 2 tokens 13.6 / 12.0, one of 16 15.2 / 14.8, one of 64 26.7 / 32.4; of 64 states: one of 16 18.5 / 25.3.
             both = self.activation(B.as_strided((*B.shape[:2], 2 * states), B.stride()), "none")
             B, C = both[:, :states], both[:, states:]
         b_at, c_at = self._sliced(B, "selective_scan B"), self._sliced(C, "selective_scan C")

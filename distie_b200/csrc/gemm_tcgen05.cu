@@ -1157,14 +1157,15 @@ extern "C" int distie_gemm_tcgen05_act(const void* x, int ldx, const void* w, vo
 // while a few pairs of CTAs walk the whole of K.  `splits` pairs share a tile's K (as many stages of 64 each but for the last
 // one) and leave slices [splits, M, N] float32 whose sum is the product, for consumers that add slices up.
 // distie_gemm_tcgen05_splits: how many slices that is; 1: not worth it (a quarter of the pairs are busy already, or a share
-// would be shorter than four stages, or K is below 704: its whole walk costs little more than a launch).  Measured, whole
-// and split, us: 1,024 x 128 x 3,072 17.5 and 5.9 (8 slices); 1,001 x 16 x 1,536 10.3 and 4.8 (6); 700 x 200 x 1,000 8.7 and
+// would be shorter than four stages, or K is 640 or less: its whole walk costs little more than a launch; or rows are wide
+// and no multiple of four floats, where a norm adds slices up in a pass of its own: product and norm of 2,048 x 250 x 704 21.2
+// whole and 24.5 split, x 1,536 25.0 and 25.8, from 2,048 of K on the split gains more).  Measured, whole and split, us: 1,024 x 128 x 3,072 17.5 and 5.9 (8 slices); 1,001 x 16 x 1,536 10.3 and 4.8 (6); 700 x 200 x 1,000 8.7 and
 // 5.4 (4); 1,500 x 250 x 1,536 (12 tiles) 18.8 and 15.7 (6).
 extern "C" int distie_gemm_tcgen05_splits(int M, int N, int K, int sm_count) {
   if (M < 2 * kGemmBM || N < 1 || K < 1 || sm_count < 2) return 1;
   const int tiles = (M + 2 * kGemmBM - 1) / (2 * kGemmBM) * ((N + 127) / 128), k_blocks = (K + kGemmBK - 1) / kGemmBK;
   int splits = min(8, min(sm_count / 2 / tiles, k_blocks / 4));
-  if (tiles > sm_count / 8 || splits < 2 || k_blocks < 11) return 1;
+  if (tiles > sm_count / 8 || splits < 2 || k_blocks < 11 || (N > 192 && (N & 3) && K < 2048)) return 1;
   const int share = (k_blocks + splits - 1) / splits;
   return (k_blocks + share - 1) / share;
 }

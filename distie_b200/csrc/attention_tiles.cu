@@ -12,6 +12,11 @@
 // Arithmetic is the size-agnostic kernel's: float32 products and sums, scores scaled (and capped) after the product,
 // accurate exponentials, the same visible keys (window, chunk, keep_first), the sink in the denominator, and a key whose
 // page the block table does not hold is reported and skipped.  Sizes: multiples of four up to 128.
+//
+// A value that is not finite reaches the tokens that see it and no others: a tile whose sums are not all finite is gone
+// through once more without the products of the keys that a row does not see (the check of the sums: nothing that shows).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace distie {
@@ -98,117 +103,134 @@ __global__ void __launch_bounds__(kTileThreads, 2) attention_tiles_kernel(TileAt
     copies_commit();
   };
 
-  find_rows(0);
 #pragma unroll
   for (int i = 0; i < kTileRows * kRowCopies / kTileThreads; ++i) {
     const int idx = i * kTileThreads + tid, r = idx / kRowCopies, e = idx % kRowCopies * 4;
     const bool live = r < rows && e < a.head_dim;
     copy_float4(&sm.q[r][e], a.q + (live ? (size_t)(t0 + r) * a.q_stride + (size_t)head * a.head_dim + e : 0), live);
   }
-  __syncthreads();
-  copy_block(0, a.k, a.head_dim, sm.k[0], TileShared<D>::kKeyPitch);
-  copy_block(0, a.v, a.value_dim, sm.v[0], D);
-
-  float o[4][kCols] = {}, m[4], l[4];
+  float o[4][kCols], m[4], l[4];
   int first[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    m[i] = -INFINITY;
-    l[i] = 0.f;
-    first[i] = first_visible_key(pos0 + rg * 4 + i, a.window, a.chunk);
-  }
-  for (int b = 0; b < blocks; ++b) {
-    const bool more = b + 1 < blocks;
-    if (more) find_rows(b + 1);
-    copies_wait<1>();  // K is here (and the queries); V may be on its way
+  for (int i = 0; i < 4; ++i) first[i] = first_visible_key(pos0 + rg * 4 + i, a.window, a.chunk);
+  // All keys of the tile.  A key that a row does not see has weight 0 there, and 0 times a value that is not finite is NaN:
+  // CAREFUL marks such weights as -0 and leaves the products out.
+  auto walk_keys = [&](auto careful) {
+    constexpr bool CAREFUL = decltype(careful)::value;
+    find_rows(0);
     __syncthreads();
-    float s[4][4] = {};
-#pragma unroll 4
-    for (int e = 0; e < D; e += 4) {
-      float4 q[4], k[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4*>(&sm.q[rg * 4 + i][e]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4*>(&sm.k[c + 16 * j][e]);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          s[i][j] = fmaf(q[i].x, k[j].x, s[i][j]);
-          s[i][j] = fmaf(q[i].y, k[j].y, s[i][j]);
-          s[i][j] = fmaf(q[i].z, k[j].z, s[i][j]);
-          s[i][j] = fmaf(q[i].w, k[j].w, s[i][j]);
-        }
-    }
-    const int start = block_start(b);
-    bool live[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) live[j] = sm.row[b & 1][c + 16 * j] >= 0;
+    copy_block(0, a.k, a.head_dim, sm.k[0], TileShared<D>::kKeyPitch);  // (and the queries)
+    copy_block(0, a.v, a.value_dim, sm.v[0], D);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int pos = pos0 + rg * 4 + i;
-      float top = m[i];
+      m[i] = -INFINITY;
+      l[i] = 0.f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int key = start + c + 16 * j;
-        const bool seen = live[j] && key <= pos && (key >= first[i] || key < a.keep_first);
-        s[i][j] = seen ? cap_score(s[i][j] * a.scale, a.softcap) : -INFINITY;  // scaled after the product
-        top = fmaxf(top, s[i][j]);
-      }
-#pragma unroll
-      for (int offset = 8; offset > 0; offset >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, offset));
-      const float base = top == -INFINITY ? 0.f : top;  // nothing seen yet: every exponential is 0
-      const float corr = expf(m[i] - base);
-      float sum = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float p = expf(s[i][j] - base);
-        sm.p[rg * 4 + i][c + 16 * j] = p;
-        sum += p;
-      }
-      l[i] = l[i] * corr + sum;  // of this thread's keys: summed over the row's threads at the end
-      m[i] = top;
-#pragma unroll
-      for (int e = 0; e < kCols; ++e) o[i][e] *= corr;
+      for (int e = 0; e < kCols; ++e) o[i][e] = 0.f;
     }
-    __syncthreads();  // K is done with
-    if (more) {
-      copy_block(b + 1, a.k, a.head_dim, sm.k[0], TileShared<D>::kKeyPitch);
-      copies_wait<1>();
-    } else {
-      copies_wait<0>();
-    }
-    __syncthreads();  // V is here
+    for (int b = 0; b < blocks; ++b) {
+      const bool more = b + 1 < blocks;
+      if (more) find_rows(b + 1);
+      copies_wait<1>();  // K is here (and the queries); V may be on its way
+      __syncthreads();
+      float s[4][4] = {};
 #pragma unroll 4
-    for (int j = 0; j < kTileKeys; j += 4) {
-      float4 p[4];
+      for (int e = 0; e < D; e += 4) {
+        float4 q[4], k[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(&sm.p[rg * 4 + i][j]);
+        for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4*>(&sm.q[rg * 4 + i][e]);
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        float v[kCols];
+        for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4*>(&sm.k[c + 16 * j][e]);
 #pragma unroll
-        for (int e = 0; e < kCols; e += kVec) {
-          const float* src = &sm.v[j + jj][kVec * c + 16 * e];
-          if (kVec == 4) {
-            const float4 x = *reinterpret_cast<const float4*>(src);
-            v[e] = x.x; v[e + 1] = x.y; v[e + (kVec > 2 ? 2 : 0)] = x.z; v[e + (kVec > 3 ? 3 : 0)] = x.w;
-          } else {
-            const float2 x = *reinterpret_cast<const float2*>(src);
-            v[e] = x.x; v[e + 1] = x.y;
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            s[i][j] = fmaf(q[i].x, k[j].x, s[i][j]);
+            s[i][j] = fmaf(q[i].y, k[j].y, s[i][j]);
+            s[i][j] = fmaf(q[i].z, k[j].z, s[i][j]);
+            s[i][j] = fmaf(q[i].w, k[j].w, s[i][j]);
+          }
+      }
+      const int start = block_start(b);
+      bool live[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) live[j] = sm.row[b & 1][c + 16 * j] >= 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int pos = pos0 + rg * 4 + i;
+        float top = m[i];
+        bool hidden[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int key = start + c + 16 * j;
+          const bool seen = live[j] && key <= pos && (key >= first[i] || key < a.keep_first);
+          hidden[j] = !seen;
+          s[i][j] = seen ? cap_score(s[i][j] * a.scale, a.softcap) : -INFINITY;  // scaled after the product
+          top = fmaxf(top, s[i][j]);
+        }
+#pragma unroll
+        for (int offset = 8; offset > 0; offset >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, offset));
+        const float base = top == -INFINITY ? 0.f : top;  // nothing seen yet: every exponential is 0
+        const float corr = expf(m[i] - base);
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float p = expf(s[i][j] - base);
+          sm.p[rg * 4 + i][c + 16 * j] = CAREFUL && hidden[j] ? -0.f : p;
+          sum += p;
+        }
+        l[i] = l[i] * corr + sum;  // of this thread's keys: summed over the row's threads at the end
+        m[i] = top;
+#pragma unroll
+        for (int e = 0; e < kCols; ++e) o[i][e] *= corr;
+      }
+      __syncthreads();  // K is done with
+      if (more) {
+        copy_block(b + 1, a.k, a.head_dim, sm.k[0], TileShared<D>::kKeyPitch);
+        copies_wait<1>();
+      } else {
+        copies_wait<0>();
+      }
+      __syncthreads();  // V is here
+#pragma unroll 4
+      for (int j = 0; j < kTileKeys; j += 4) {
+        float4 p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(&sm.p[rg * 4 + i][j]);
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+          float v[kCols];
+#pragma unroll
+          for (int e = 0; e < kCols; e += kVec) {
+            const float* src = &sm.v[j + jj][kVec * c + 16 * e];
+            if (kVec == 4) {
+              const float4 x = *reinterpret_cast<const float4*>(src);
+              v[e] = x.x; v[e + 1] = x.y; v[e + (kVec > 2 ? 2 : 0)] = x.z; v[e + (kVec > 3 ? 3 : 0)] = x.w;
+            } else {
+              const float2 x = *reinterpret_cast<const float2*>(src);
+              v[e] = x.x; v[e + 1] = x.y;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float w = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
+            if (CAREFUL && __float_as_uint(w) == 0x80000000u) continue;
+#pragma unroll
+            for (int e = 0; e < kCols; ++e) o[i][e] = fmaf(w, v[e], o[i][e]);
           }
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float w = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
-#pragma unroll
-          for (int e = 0; e < kCols; ++e) o[i][e] = fmaf(w, v[e], o[i][e]);
-        }
       }
+      __syncthreads();
+      if (more) copy_block(b + 1, a.v, a.value_dim, sm.v[0], D);
     }
-    __syncthreads();
-    if (more) copy_block(b + 1, a.v, a.value_dim, sm.v[0], D);
-  }
+  };
+  walk_keys(std::false_type{});
+  float odd = 0.f;  // NaN when a sum is not finite: then once more, row by row only what it sees
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int e = 0; e < kCols; ++e) odd += 0.f * o[i][e];
+  if (__syncthreads_or(odd != 0.f)) walk_keys(std::true_type{});
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
 #pragma unroll

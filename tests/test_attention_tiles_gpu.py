@@ -92,3 +92,46 @@ def test_a_missing_page_is_reported_and_its_keys_skipped():
     assert torch.isfinite(out).all()
     ks.attention(q, out, step, kv, 1, 1, 64, 8, 0.125)  # the page lies before every row's window
     ks.check_errors()
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("where,window,keep_first", [(150, None, 0), (70, 40, 0), (3, 40, 5), (2, 40, 2), (99, 1, 0)])
+def test_a_value_that_is_not_finite_reaches_the_tokens_that_see_it_alone(where, window, keep_first, bad):
+    """The key's tile holds rows before it, behind it and, with a window, past it; the first keys are kept for good or not."""
+    from distie_b200.kernels import make_kernels
+
+    ks = make_kernels(torch.float32, "cuda:0")
+    past, n, heads, dim = 60, 130, 2, 64
+    kv = make_cache(torch.float32, 16, 1, 16, dim, 1, 16)
+    step = step_of([n], [past], [0])
+    generator = torch.Generator(device="cuda").manual_seed(4)
+    q = torch.randn(n, heads * dim, generator=generator, device="cuda")
+    page, slot = kv.block_table[0].long()[where // 16], where % 16
+    kv.v[page, 0, slot] = 0.0
+    want = exact(q, kv, [n], [past], heads, 1, dim, 0.125, window, None, keep_first, 0.0, None)
+    kv.v[page, 0, slot, 5] = bad
+    out = torch.empty(n, heads * dim, device="cuda")
+    ks.attention(q, out, step, kv, heads, 1, dim, window, 0.125, None, keep_first)
+    ks.check_errors()
+    assert ks.kernel_counts.get("attention_tiles")
+    position = torch.arange(past, past + n, device="cuda")
+    sees = (position >= where) & ((position - where < (window or 10**6)) | (where < keep_first))
+    spoiled = torch.zeros(n, heads, dim, dtype=torch.bool, device="cuda")
+    spoiled[sees, :, 5] = True
+    spoiled = spoiled.view(n, -1)
+    assert torch.equal(~torch.isfinite(out), spoiled)
+    error = float((out.double() - want)[~spoiled].norm() / want[~spoiled].norm())
+    assert error <= BOUND, f"off by {error:.2e}"
+
+
+def test_a_key_that_is_not_finite_reaches_the_tokens_that_see_it_alone():
+    from distie_b200.kernels import make_kernels
+
+    ks = make_kernels(torch.float32, "cuda:0")
+    kv = make_cache(torch.float32, 8, 1, 16, 64, 1, 8)
+    step = step_of([100], [20], [0])
+    q, out, clean = (torch.randn(100, 64, generator=torch.Generator(device="cuda").manual_seed(5 + i), device="cuda") for i in range(3))
+    ks.attention(q, clean, step, kv, 1, 1, 64, None, 0.125)
+    kv.k[kv.block_table[0].long()[80 // 16], 0, 80 % 16, 3] = float("nan")
+    ks.attention(q, out, step, kv, 1, 1, 64, None, 0.125)
+    assert torch.equal(out[:60], clean[:60]) and not torch.isfinite(out[60:]).any()

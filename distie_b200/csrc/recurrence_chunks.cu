@@ -22,7 +22,8 @@
 // in the six products of weight 2^-16 and more.  The largest one (high x high) has accumulators of its own: the tensor
 // core truncates when it accumulates, and so truncates 4 or 8 times into a sum at full size instead of 24 or 48 times.
 // Decays are products of the g, as in the walk, never differences of logarithms, so a decay of 0 is a 0.
-// (A value that is not finite spoils the whole chunk of its request, as it spoils all later tokens in the walk.)
+// A number that is not finite spoils what the walk lets it spoil, its own token and those behind it: chunk_read takes a chunk
+// whose sums are not all finite token by token (walk_chunk).  (The state behind it may hold NaN where the walk's holds an infinity.)
 //
 // Why chunks: the walk is a chain of about 110 dependent instructions a token and head column, 0.15 to 0.25 us a token
 // whatever the machine could do beside it.  Single tokens, short portions and many portions of small states, which fill the
@@ -785,13 +786,70 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(ChunkArgs a
   store_state(slot);
 }
 
+// The read-outs of a chunk token by token, as the walk of recurrent.cu takes them, from the state before the chunk: what
+// chunk_read does when a sum of its products is not finite.  A product with a weight of 0 for a token that a row does not see is NaN
+// when that token's numbers are not finite; here a row meets nothing behind it.  A warp a value element, the state's column
+// over its lanes.  Every thread of the block calls it; reads_s: rows * value_dim floats.
+template <int RULE>
+__device__ __noinline__ void walk_chunk(const ChunkArgs& a, const Decays& d, float* reads_s, int chunk, int head, int t0, int rows) {
+  const int lane = threadIdx.x & 31, group = head / (a.heads / a.groups);
+  const float skip = RULE == kRuleSsd && a.skip ? a.skip[head] : 0.f;
+  for (int j = threadIdx.x >> 5; j < a.value_dim; j += kWideThreads / 32) {
+    const float* column = a.chunks + (((size_t)chunk * a.heads + head) * a.value_dim + j) * a.key_dim;
+    float S[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) S[r] = lane + 32 * r < a.key_dim ? column[lane + 32 * r] : 0.f;
+    for (int t = 0; t < rows; ++t) {
+      const float* q_row = a.q + (size_t)(t0 + t) * a.q_stride + group * a.key_dim;
+      const float* k_row = a.k + (size_t)(t0 + t) * a.k_stride + group * a.key_dim;
+      float q[4], k[4], qq = 0.f, kk = 0.f;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const bool live = lane + 32 * r < a.key_dim;
+        q[r] = live ? q_row[lane + 32 * r] : 0.f;
+        k[r] = live ? k_row[lane + 32 * r] : 0.f;
+        qq += q[r] * q[r];
+        kk += k[r] * k[r];
+      }
+      if (RULE == kRuleDelta) {
+        qq = rsqrtf((float)a.key_dim) / sqrtf(warp_sum(qq) + 1e-6f);
+        kk = 1.f / sqrtf(warp_sum(kk) + 1e-6f);
+      }
+      float kq = 0.f, sum_k = 0.f, sum_q = 0.f;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        if (RULE == kRuleDelta) q[r] *= qq, k[r] *= kk;
+        if (RULE == kRuleGated) q[r] *= a.q_scale;
+        kq += k[r] * q[r];
+        sum_k += S[r] * k[r];
+        sum_q += S[r] * q[r];
+      }
+      const float g = d.g[t], factor = d.factor[t], v = j < a.v_dim ? a.v[(size_t)(t0 + t) * a.v_stride + (size_t)head * a.v_dim + j] : 1.f;
+      const float u = RULE == kRuleDelta ? factor * (v - g * warp_sum(sum_k)) : factor * v;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) S[r] = g * S[r] + k[r] * u;
+      const float read = g * warp_sum(sum_q) + u * warp_sum(kq);
+      if (lane == 0) reads_s[t * a.value_dim + j] = RULE == kRuleSsd ? read + skip * v : read;
+    }
+  }
+  __syncthreads();
+  const bool divided = RULE == kRuleGated && a.floor;
+  const int columns = divided ? a.v_dim : a.value_dim;
+  for (int idx = threadIdx.x; idx < rows * columns; idx += kWideThreads) {
+    const int t = idx / columns, j = idx % columns;
+    float x = reads_s[t * a.value_dim + j];
+    if (divided) x /= fmaxf(fabsf(reads_s[t * a.value_dim + a.v_dim]), a.floor[(size_t)(t0 + t) * a.heads + head]) + 1e-6f;
+    a.out[(size_t)(t0 + t) * a.out_stride + (size_t)head * columns + j] = x;
+  }
+}
+
 // O of a chunk from its own tokens and the state before it.  Shared memory: Q | K | S, then Q | the scores | U.
 using StateTriple = Triple<kKeyPitch, 144>;
 constexpr size_t read_shared(int value_dim) {  // (parts of S and U lie as for 144 values where there are more than 128)
   return 2 * KeyTriple::kBytes + (value_dim > 128 ? StateTriple::kBytes : Triple<kKeyPitch, 128>::kBytes);
 }
 template <int RULE, int VALUES>
-__global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a) {
+__global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(const __grid_constant__ ChunkArgs a) {
   extern __shared__ __align__(128) unsigned char chunk_s[];
   __shared__ Decays d;
   int t0;
@@ -888,6 +946,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a
   float* out = a.out + (size_t)t0 * a.out_stride + (size_t)head * columns;
   const bool pairs = (columns & 1) == 0 && (a.out_stride & 1) == 0 && ((uintptr_t)a.out & 7) == 0;
   const auto p_at = first_rows(p, rg * 16, lane);
+  float odd = 0.f;  // NaN when a sum is not finite
 #pragma unroll
   for (int i = 0; i < kUnits; ++i) {
     const int unit = cq + 4 * i;
@@ -905,16 +964,20 @@ __global__ void __launch_bounds__(kWideThreads, 1) chunk_read_kernel(ChunkArgs a
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         o[i][n][r] += acc.of(n, r);
-        if (divided && unit * 16 + 8 * n + 2 * c + (r & 1) == a.v_dim) d.g[row0 + 8 * (r >> 1)] = o[i][n][r];  // (the g are done with)
+        odd += 0.f * o[i][n][r];
+        if (divided && unit * 16 + 8 * n + 2 * c + (r & 1) == a.v_dim) d.suf[row0 + 8 * (r >> 1)] = o[i][n][r];  // (done with)
       }
+  }
+  if (__syncthreads_or(odd != 0.f)) {
+    walk_chunk<RULE>(a, d, reinterpret_cast<float*>(chunk_s), blockIdx.y, head, t0, rows);
+    return;
   }
   float over[2] = {1.f, 1.f};
   if (divided) {
-    __syncthreads();
 #pragma unroll
     for (int h = 0; h < 2; ++h)
       if (row0 + 8 * h < rows)
-        over[h] = fmaxf(fabsf(d.g[row0 + 8 * h]), a.floor[(size_t)(t0 + row0 + 8 * h) * a.heads + head]) + 1e-6f;
+        over[h] = fmaxf(fabsf(d.suf[row0 + 8 * h]), a.floor[(size_t)(t0 + row0 + 8 * h) * a.heads + head]) + 1e-6f;
   }
 #pragma unroll
   for (int i = 0; i < kUnits; ++i) {

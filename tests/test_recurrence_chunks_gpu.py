@@ -102,3 +102,48 @@ def test_chunks_of_a_recurrence(rule, strong, lengths, heads, groups, key_dim, v
     for name, a, b in (("read-out", got, want), ("state", state, want_state)):
         error = float((a.double() - b).norm() / b.norm())
         assert error <= BOUND, f"{rule} {name}: off by {error:.2e}"
+
+
+def inputs(rule, lengths, heads, groups, key_dim, value_dim, seed=7):
+    generator = torch.Generator(device="cuda").manual_seed(seed)
+    normal = lambda *shape: torch.randn(*shape, generator=generator, device="cuda")  # noqa: E731
+    total = sum(lengths)
+    p = {"q": normal(total, groups * key_dim), "k": normal(total, groups * key_dim) + 0.3, "v": normal(total, heads * value_dim),
+         "decay": normal(total, heads), "write": normal(total, heads), "rate": normal(heads) * 0.5, "bias": normal(heads) - 3,
+         "skip": normal(heads) if rule == "ssd" else None, "state": normal(len(lengths), heads, value_dim, key_dim)}
+    if rule == "gated":
+        p["decay"], p["write"] = torch.exp(-p["decay"] ** 2 * 0.02), torch.sigmoid(p["write"])
+    return p
+
+
+def run(ks, rule, p, lengths, heads, groups, key_dim, value_dim, state=None):
+    state = p["state"].clone() if state is None else state
+    got = ks.linear_recurrence(rule, p["q"], p["k"], p["v"], p["decay"], p["write"], state,
+                               step_of(lengths, [3] * len(lengths), list(range(len(lengths)))), heads, groups, key_dim, value_dim,
+                               decay_rate=p["rate"], decay_bias=p["bias"] if rule != "gated" else None, skip=p["skip"])
+    ks.check_errors()
+    assert "recurrence_chunks" in ks.kernel_counts and "linear_recurrence" not in ks.kernel_counts
+    return got, state
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["q", "k", "v", "decay", "write", "state"])
+@pytest.mark.parametrize("rule", ["delta", "ssd", "gated"])
+def test_a_number_that_is_not_finite_spoils_its_token_and_those_behind_it(rule, where, bad):
+    """As in the walk: nothing before the token, no other request, no column of a state that does not meet it."""
+    from distie_b200.kernels import make_kernels
+
+    ks = make_kernels(torch.bfloat16, "cuda:0")
+    lengths, heads, groups, key_dim, value_dim = [300, 257, 200], 4, 2, 64, 48
+    p = inputs(rule, lengths, heads, groups, key_dim, value_dim)
+    if where == "state":
+        p["state"][0, 1, 5, 7] = bad
+    else:
+        p[where][100, 1], p[where][300 + 256, 0] = bad, bad  # inside a chunk; the last token of a request
+    want, want_state = exact(rule, p, lengths, range(3), heads, groups, key_dim, value_dim, False)
+    got, state = run(ks, rule, p, lengths, heads, groups, key_dim, value_dim)
+    for name, a, b in (("read-out", got, want), ("state", state, want_state)):
+        fine = torch.isfinite(b)
+        assert fine.any() and torch.equal(torch.isfinite(a), fine), f"{name}: other numbers are spoiled"
+        error = float((a.double() - b)[fine].norm() / b[fine].norm())
+        assert error <= BOUND, f"{name}: off by {error:.2e}"

@@ -35,7 +35,7 @@ _CLUSTER_SPLITS = 8             # splits of a decode attention that one cluster 
 _TENSOR_CORE_ROWS = 128         # from here on the tcgen05 kernel's 128-row tiles are full; in between: the library
 _MAX_TERMS = 24                 # terms of a pending sum that the layer-norm kernel adds up itself
 _RULES = {"delta": 0, "ssd": 1, "gated": 2}
-_CHUNK_BYTES = 1 << 30          # the most that the states between the chunks of a step may take
+_CHUNK_BYTES = 512 << 20        # the most that the states between the chunks of tiles that run together may take
 _ACTS = {"relu2": 1, "gelu": 2, "xielu": 3}
 _SCORINGS = {"sigmoid": 0, "softmax": 1, "softmax_chosen": 2}
 _PLAIN_ACTS = {"none": 0, "silu": 1, "tanh": 2}
@@ -737,17 +737,8 @@ class DeviceKernels(KernelSet):
         ]
         tokens, seqs = step.num_tokens, step.num_seqs  # what the walk takes
         if self._in_chunks(rule, state, step, heads, key_dim, value_dim):
-            floats = function("distie_recurrence_chunks_scratch_floats")(_RULES[rule], step.num_q_tiles, heads, key_dim, value_dim)
-            chunks = torch.empty(floats, dtype=torch.float32, device=q.device)
-            check(
-                function("distie_recurrence_chunks")(
-                    *head, chunks.data_ptr(), step.q_tiles.data_ptr(), step.num_q_tiles, step.token_seq.data_ptr(),
-                    step.seq_seat.data_ptr(), heads, groups, key_dim, value_dim, int(bool(unit_column)),
-                    1.0, None, self.error_flag.data_ptr(), self._stream(),
-                ),
-                "recurrence_chunks",
-            )
-            self._ran("recurrence_chunks", 3)
+            tail = [heads, groups, key_dim, value_dim, int(bool(unit_column)), 1.0, None]
+            self._run_chunks(rule, head, tail, step, heads, key_dim, value_dim)
             tokens = seqs = step.num_decode_tokens  # single tokens come first in a step
         if tokens:
             scratch = torch.empty(tokens * (2 * heads + groups), dtype=torch.float32, device=q.device)
@@ -772,20 +763,31 @@ class DeviceKernels(KernelSet):
             raise KernelError("stabilized_memory: contiguous gates are expected")
         columns, base = heads * key_dim, rows.data_ptr()
         out = torch.empty((step.num_tokens, heads * value_dim), dtype=torch.float32, device=rows.device)
-        floats = function("distie_recurrence_chunks_scratch_floats")(_RULES["gated"], step.num_q_tiles, heads, key_dim, value_dim + 1)
-        chunks = torch.empty(floats, dtype=torch.float32, device=rows.device)
-        check(
-            function("distie_recurrence_chunks")(
-                _RULES["gated"], base, rows.stride(0), base + 4 * columns, rows.stride(0), base + 8 * columns, rows.stride(0),
-                keep.data_ptr(), heads, take.data_ptr(), heads, 1, 0, None, None, None, state.data_ptr(), out.data_ptr(),
-                out.stride(0), chunks.data_ptr(), step.q_tiles.data_ptr(), step.num_q_tiles, step.token_seq.data_ptr(),
-                step.seq_seat.data_ptr(), heads, heads, key_dim, value_dim + 1, 1, float(q_scale), floor.data_ptr(),
-                self.error_flag.data_ptr(), self._stream(),
-            ),
-            "recurrence_chunks",
-        )
-        self._ran("recurrence_chunks", 3)
+        head = [
+            _RULES["gated"], base, rows.stride(0), base + 4 * columns, rows.stride(0), base + 8 * columns, rows.stride(0),
+            keep.data_ptr(), heads, take.data_ptr(), heads, 1, 0, None, None, None, state.data_ptr(), out.data_ptr(), out.stride(0),
+        ]
+        tail = [heads, heads, key_dim, value_dim + 1, 1, float(q_scale), floor.data_ptr()]
+        self._run_chunks("gated", head, tail, step, heads, key_dim, value_dim + 1)
         return out
+
+    def _run_chunks(self, rule, head, tail, step, heads, key_dim, value_dim) -> None:
+        """The tiles of a step in groups whose scratch stays within _CHUNK_BYTES, one after another in one buffer: the chain
+        reads and writes the requests' states, so a group may start at any tile.  (Delta rule, 28 heads of 128: a group is
+        6,200 tokens.)"""
+        of_tile = function("distie_recurrence_chunks_scratch_floats")(_RULES[rule], 1, heads, key_dim, value_dim)
+        count = -(-step.num_q_tiles // min(32767, _CHUNK_BYTES // (4 * of_tile)))
+        size = -(-step.num_q_tiles // count)
+        chunks = torch.empty(size * of_tile, dtype=torch.float32, device=self.device)
+        for first in range(0, step.num_q_tiles, size):
+            check(
+                function("distie_recurrence_chunks")(
+                    *head, chunks.data_ptr(), step.q_tiles.data_ptr() + 8 * first, min(size, step.num_q_tiles - first),
+                    step.token_seq.data_ptr(), step.seq_seat.data_ptr(), *tail, self.error_flag.data_ptr(), self._stream(),
+                ),
+                "recurrence_chunks",
+            )
+            self._ran("recurrence_chunks", 3)
 
     def _in_chunks(self, rule, state, step, heads, key_dim, value_dim) -> bool:
         """Whether the portions of a step run in chunks of 64 tokens instead of token by token (16-bit engine: the
@@ -794,9 +796,8 @@ class DeviceKernels(KernelSet):
         portions, rest = step.num_seqs - singles, step.num_tokens - singles
         return (self.dtype == torch.bfloat16 and portions > 0 and step.num_q_tiles > 0
                 and key_dim <= 128 and value_dim <= 144 and chunks_pay(rule, rest, portions, heads, key_dim, value_dim)
-                and step.num_q_tiles <= 32767 and state.is_contiguous()
-                and 4 * function("distie_recurrence_chunks_scratch_floats")(_RULES[rule], step.num_q_tiles, heads, key_dim,
-                                                                            value_dim) <= _CHUNK_BYTES)
+                and state.is_contiguous()
+                and 4 * function("distie_recurrence_chunks_scratch_floats")(_RULES[rule], 1, heads, key_dim, value_dim) <= _CHUNK_BYTES)
 
     def gated_rmsnorm(self, x, gate, weight, eps, group, gate_first, out, activation="silu") -> None:
         self._rows32(x, "gated_rmsnorm x")

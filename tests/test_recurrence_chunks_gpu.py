@@ -147,3 +147,20 @@ def test_a_number_that_is_not_finite_spoils_its_token_and_those_behind_it(rule, 
         assert fine.any() and torch.equal(torch.isfinite(a), fine), f"{name}: other numbers are spoiled"
         error = float((a.double() - b)[fine].norm() / b[fine].norm())
         assert error <= BOUND, f"{name}: off by {error:.2e}"
+
+
+@pytest.mark.parametrize("rule", ["delta", "ssd", "gated"])
+def test_portions_beyond_the_scratch_run_in_groups_of_tiles(rule, monkeypatch):
+    """Groups that end inside a request and between two: the same arithmetic, so the same numbers."""
+    from distie_b200.kernels import device, make_kernels
+
+    lengths, heads, groups, key_dim, value_dim = [640, 300, 385, 140], 4, 2, 64, 48
+    p = inputs(rule, lengths, heads, groups, key_dim, value_dim)  # 5 + 3 + 4 + 2 tiles
+    whole, whole_state = run(make_kernels(torch.bfloat16, "cuda:0"), rule, p, lengths, heads, groups, key_dim, value_dim)
+    of_tile = device.function("distie_recurrence_chunks_scratch_floats")(device._RULES[rule], 1, heads, key_dim, value_dim)
+    for tiles in (1, 3, 13):
+        monkeypatch.setattr(device, "_CHUNK_BYTES", 4 * of_tile * tiles + 3)
+        ks = make_kernels(torch.bfloat16, "cuda:0")
+        got, state = run(ks, rule, p, lengths, heads, groups, key_dim, value_dim)
+        assert ks.kernel_counts["recurrence_chunks"] == -(-14 // tiles)
+        assert torch.equal(got, whole) and torch.equal(state, whole_state)

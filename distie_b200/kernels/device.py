@@ -155,6 +155,10 @@ class DeviceKernels(KernelSet):
     def add_rmsnorm(self, delta, residual, weight, eps, out, rows_index=None) -> None:
         rows = out.shape[0]
         rows_ptr = rows_index.data_ptr() if rows_index is not None else None
+        if delta is not None and delta.dim() == 2 and delta.dtype != self.dtype:
+            if delta.dtype != torch.float32:
+                raise KernelError(f"add_rmsnorm: a matrix of {self.dtype} or float32 is expected, not of {delta.dtype}")
+            delta = delta.contiguous().unsqueeze(0)  # (a sum of terms: one float32 slice)
         if delta is not None and delta.dim() == 3:
             code = function("distie_add_rmsnorm_split")(
                 delta.data_ptr(), delta.shape[0], delta.stride(0), residual.data_ptr(), weight.data_ptr(),

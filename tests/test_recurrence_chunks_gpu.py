@@ -164,3 +164,67 @@ def test_portions_beyond_the_scratch_run_in_groups_of_tiles(rule, monkeypatch):
         got, state = run(ks, rule, p, lengths, heads, groups, key_dim, value_dim)
         assert ks.kernel_counts["recurrence_chunks"] == -(-14 // tiles)
         assert torch.equal(got, whole) and torch.equal(state, whole_state)
+
+
+@pytest.mark.parametrize("rule", ["delta", "ssd", "gated"])
+@pytest.mark.parametrize("slices,offset,extra", [(3, 0, 0), (1, 1, 3), (3, 1, 0)])
+def test_slices_and_addresses_that_no_vector_fits(rule, slices, offset, extra):
+    """Decay and write as slices of one projection; rows of q, k and v and the state a float off 16 bytes, rows of any stride.
+    Adding up three slices rounds twice more, in a gate that a chunk multiplies up to 64 times: twice the bound."""
+    from distie_b200.kernels import make_kernels
+
+    ks = make_kernels(torch.bfloat16, "cuda:0")
+    lengths, heads, groups, key_dim, value_dim = [300, 257, 200], 4, 2, 64, 48
+    p = inputs(rule, lengths, heads, groups, key_dim, value_dim)
+    total, columns = sum(lengths), 2 * groups * key_dim + heads * value_dim
+    rows = torch.full((total, offset + columns + extra), float("nan"), device="cuda")[:, offset : offset + columns]
+    rows.copy_(torch.cat([p["q"], p["k"], p["v"]], -1))
+    p["q"], p["k"], p["v"] = rows.split([groups * key_dim, groups * key_dim, heads * value_dim], -1)
+    both = torch.cat([p["decay"], p["write"]], -1)
+    gates = torch.empty(slices, total, 2 * heads + 1, device="cuda")[:, :, : 2 * heads]
+    for s in range(1, slices):
+        gates[s] = both * (0.2 * s)
+    gates[0] = both - gates[1:].sum(0)
+    if rule == "gated":  # (a decay stays what it was: at most 1)
+        gates[0, :, :heads] = torch.minimum(gates[0, :, :heads], 1 - gates[1:, :, :heads].sum(0))
+    summed = gates.double().sum(0)
+    held = torch.empty(p["state"].numel() + offset, device="cuda")[offset:].view_as(p["state"]).copy_(p["state"])
+    want, want_state = exact(rule, p | {"decay": summed[:, :heads], "write": summed[:, heads:]}, lengths, range(3), heads, groups,
+                             key_dim, value_dim, False)
+    p["decay"], p["write"] = gates[:, :, :heads], gates[:, :, heads:]
+    got, state = run(ks, rule, p, lengths, heads, groups, key_dim, value_dim, held)
+    for name, a, b in (("read-out", got, want), ("state", state, want_state)):
+        error = float((a.double() - b).norm() / b.norm())
+        assert error <= (2 if slices > 1 else 1) * BOUND, f"{name}: off by {error:.2e}"
+
+
+@pytest.mark.parametrize("lengths,heads,key_dim,value_dim", [([917], 2, 128, 128), ([513, 64, 700], 3, 64, 143), ([400, 333], 4, 128, 40)])
+@pytest.mark.parametrize("offset,extra", [(0, 0), (1, 2)])
+def test_a_stabilised_memory_in_one_go(lengths, heads, key_dim, value_dim, offset, extra):
+    """The projection as it is: q scaled on the way in, read-outs divided on the way out, by the normaliser in some rows
+    and by the floor in others.  A divisor is at least 0.3 of the normaliser's size, so its error counts up to 1 / 0.3 times."""
+    from distie_b200.kernels import make_kernels
+
+    ks = make_kernels(torch.bfloat16, "cuda:0")
+    generator = torch.Generator(device="cuda").manual_seed(17)
+    normal = lambda *shape: torch.randn(*shape, generator=generator, device="cuda")  # noqa: E731
+    total, columns, scale = sum(lengths), heads * (2 * key_dim + value_dim), key_dim**-0.5
+    rows = torch.full((total, offset + columns + extra), float("nan"), device="cuda")[:, offset : offset + columns]
+    rows.copy_(normal(total, columns))
+    keep, take = torch.exp(-normal(total, heads) ** 2 * 0.02), torch.sigmoid(normal(total, heads))
+    state = normal(len(lengths), heads, value_dim + 1, key_dim)
+    q, k, v = rows.split([heads * key_dim, heads * key_dim, heads * value_dim], -1)
+    read, want_state = exact("gated", {"q": q.double() * scale, "k": k, "v": v, "decay": keep, "write": take, "state": state}, lengths,
+                             range(len(lengths)), heads, heads, key_dim, value_dim + 1, True)
+    read = read.view(total, heads, value_dim + 1)
+    size = read[:, :, value_dim].abs()
+    floor = (size * torch.where(normal(total, heads) > 0, 1.5, 0.5)).clamp_min(0.3 * float(size.square().mean().sqrt())).float()
+    assert 0.3 < float((floor > size).float().mean()) < 0.8
+    want = (read[:, :, :value_dim] / (torch.maximum(size, floor.double()) + 1e-6)[:, :, None]).reshape(total, -1)
+    step = step_of(lengths, [3] * len(lengths), list(range(len(lengths))))
+    got = ks.stabilized_memory(rows, scale, keep, take, floor, state, step, heads, key_dim, value_dim)
+    ks.check_errors()
+    assert "recurrence_chunks" in ks.kernel_counts and not {"linear_recurrence", "stabilized_readout"} & set(ks.kernel_counts)
+    for name, a, b, bound in (("read-out", got, want, (1 + 1 / 0.3) * BOUND), ("state", state, want_state, BOUND)):
+        error = float((a.double() - b).norm() / b.norm())
+        assert error <= bound, f"{name}: off by {error:.2e}"

@@ -2,12 +2,14 @@
 //
 // The size-agnostic kernel (attention_generic.cu) takes a token and a head a block: every key and value is read for every
 // token, and a key costs a warp a sum across its lanes.  Here a block keeps 32 queries in shared memory, takes the keys 64
-// at a time and holds 4 x 4 scores and 4 x D/16 outputs a thread, so that 16 (32) multiply-adds follow four (six) reads of
-// 16 bytes.  What bounds it is the FMA pipe (74 TFLOP/s) and, at 70 % of that time, the reads of shared memory; the keys of
+// at a time and holds 4 x 4 scores and 4 x D/16 outputs a thread: eight reads of 16 bytes feed 64 multiply-adds of the
+// scores, twelve (D = 128) feed 128 of the outputs.  The FMA pipe (74 TFLOP/s) is the ceiling, of which 38 % is reached (28 TFLOP/s
+// of the visible half, 1,100 tokens); the reads of shared memory take 70 % of the pipe's time beside it, and the rest goes
+// to four barriers a block of keys, the softmax between the two products and the hidden half of diagonal blocks.  The keys of
 // the next block are copied while this one's values are multiplied, and the other way round (cp.async).  Tiles of 32 rows
 // and not 64 or 128: prompts of a few hundred tokens would not fill the machine, and a causal tile's time grows with its
 // last position.  Layer of two prompts of 339 and 438 tokens, 12 heads of 128: 449 -> 61 us; 1,100 tokens, 28 heads:
-// 3,567 -> 308 us (28 TFLOP/s of the visible half).
+// 3,567 -> 308 us.  Which portions are worth a tile: tiles_pay in kernels/device.py.
 //
 // Arithmetic is the size-agnostic kernel's: float32 products and sums, scores scaled (and capped) after the product,
 // accurate exponentials, the same visible keys (window, chunk, keep_first), the sink in the denominator, and a key whose

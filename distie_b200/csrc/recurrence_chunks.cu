@@ -17,6 +17,10 @@
 //   chunk_walk   U = U_0 - W S, S <- G(end) S + K'^T U, chunk after chunk                  (a block per head and 16 values)
 //   chunk_read   as above
 //
+// The steps are the published ones: chunks of state-space duality after Dao and Gu, "Transformers are SSMs" (2024), the delta
+// rule's inverse and its W and U after Yang et al., "Parallelizing Linear Transformers with the Delta Rule over Sequence
+// Length" and "Gated Delta Networks" (both 2024).
+//
 // Precision.  The state and everything around it is float32, so the products have to be as good as float32: each operand
 // enters the tensor cores (mma.sync.m16n8k16, float32 accumulators) as three bfloat16 parts whose sum is the float32 value,
 // in the six products of weight 2^-16 and more.  The largest one (high x high) has accumulators of its own: the tensor

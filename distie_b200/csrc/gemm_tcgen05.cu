@@ -1160,7 +1160,8 @@ extern "C" int distie_gemm_tcgen05_act(const void* x, int ldx, const void* w, vo
 // would be shorter than four stages, or K is 640 or less: its whole walk costs little more than a launch; or rows are wide
 // and no multiple of four floats, where a norm adds slices up in a pass of its own: product and norm of 2,048 x 250 x 704 21.2
 // whole and 24.5 split, x 1,536 25.0 and 25.8, from 2,048 of K on the split gains more).  Measured, whole and split, us: 1,024 x 128 x 3,072 17.5 and 5.9 (8 slices); 1,001 x 16 x 1,536 10.3 and 4.8 (6); 700 x 200 x 1,000 8.7 and
-// 5.4 (4); 1,500 x 250 x 1,536 (12 tiles) 18.8 and 15.7 (6).
+// 5.4 (4); 1,500 x 250 x 1,536 (12 tiles) 18.8 and 15.7 (6).  With the norm that adds the slices up, at the edges of the rule: 256 x
+// 1,536 x 648 9.7 and 9.1; 700 x 768 (18 tiles) x 648 10.0 and 9.6, x 1,536 13.9 and 12.0; 256 x 1,536 x 1,536 13.5 and 12.7.
 extern "C" int distie_gemm_tcgen05_splits(int M, int N, int K, int sm_count) {
   if (M < 2 * kGemmBM || N < 1 || K < 1 || sm_count < 2) return 1;
   const int tiles = (M + 2 * kGemmBM - 1) / (2 * kGemmBM) * ((N + 127) / 128), k_blocks = (K + kGemmBK - 1) / kGemmBK;

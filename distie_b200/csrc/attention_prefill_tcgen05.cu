@@ -48,6 +48,7 @@
 // Sizes: keys of up to DK = 64 or 128 elements and values of up to DV = 64 or 128, multiples of 8 and of one another
 // independent.  A head smaller than its tile is padded on the way in: the copies fill what lies past the end of a key's
 // or value's row with zeros.  (The columns of Q past the head's end hold the next head's: they meet the zeros of K.)
+#include "softmax_pairs.cuh"
 #include "tcgen05.cuh"
 
 namespace distie {
@@ -87,38 +88,6 @@ struct AttnShared {
   uint32_t tmem_base;
   uint32_t failed;
 };
-
-__device__ __forceinline__ float exp2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// The softmax warps are bound by the number of instructions they issue (two warps to a scheduler, long chains of
-// dependent operations), so the loop over a block's scores uses the forms that do two things at once: the maximum
-// of three values, and float32 arithmetic on pairs of values in a 64-bit register (same rounding per value).
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
-  uint64_t v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-  return v;
-}
-__device__ __forceinline__ void halves_of(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fma_pairs(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t add_pairs(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 
 template <int DK, int DV, bool FLAT>
 __global__ void __launch_bounds__(kAttnThreads, 1)

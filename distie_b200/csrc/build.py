@@ -45,7 +45,8 @@ CUDA_UNITS: dict[str, list[str]] = {
     "base": ["elementwise.cu", "normed_residual.cu", "attention_generic.cu", "attention_tiles.cu", "attention_decode.cu",
              "sampling.cu"],
     # bfloat16 serving only: tensor-core attention for prompts, weight-streaming products for decoding
-    "bf16": ["attention_prefill.cu", "attention_decode_mma.cu", "gemm_tcgen05.cu", "attention_prefill_tcgen05.cu"],
+    "bf16": ["attention_prefill.cu", "attention_decode_mma.cu", "gemm_tcgen05.cu", "attention_prefill_tcgen05.cu",
+             "attention_prefill_pairs.cu"],
     # models with layer norms, gated heads, short convolutions or linear recurrences (both dtypes)
     "state": ["recurrent.cu", "recurrence_chunks.cu", "retention.cu"],
     # models with recurrences whose decay varies by channel (both dtypes); a unit of its own because it takes minutes
@@ -55,7 +56,7 @@ CUDA_UNITS: dict[str, list[str]] = {
     # models whose attention reads one latent row per token; gated and squared-ReLU activations on float32 products
     "latent": ["latent.cu", "latent_attention_mma.cu"],
 }
-_HEADERS = ["common.cuh", "recurrent.cuh", "tcgen05.cuh", "no_alloc.h"]
+_HEADERS = ["common.cuh", "recurrent.cuh", "tcgen05.cuh", "softmax_pairs.cuh", "no_alloc.h"]
 
 
 class BuildError(RuntimeError):

@@ -45,6 +45,7 @@ class StepLayout:
     max_kv_len: int
     packed: np.ndarray  # int32: token_ids | positions | token_seq | seq_seat | logit_rows | q_tiles
     num_q_tiles: int = 0
+    portions: list = field(default_factory=list)  # (cached tokens, new tokens) of the entries of more than one token
 
 
 def lay_out(entries: Sequence[BatchEntry], vocab_size: int | None = None) -> StepLayout:
@@ -92,7 +93,8 @@ def lay_out(entries: Sequence[BatchEntry], vocab_size: int | None = None) -> Ste
             at += 1
     if vocab_size is not None and total and (ids.min() < 0 or ids.max() >= vocab_size):
         raise ValueError(f"token id outside [0, {vocab_size})")
-    return StepLayout(seqs, total, len(entries), decode_tokens, rows, max_kv, packed, len(tiles))
+    portions = [(s.past_len, s.q_len) for s in seqs if s.q_len > 1]
+    return StepLayout(seqs, total, len(entries), decode_tokens, rows, max_kv, packed, len(tiles), portions)
 
 
 class StepStaging:
@@ -139,4 +141,5 @@ def views(buffer: torch.Tensor, layout: StepLayout) -> tuple[StepTensors, torch.
     if layout.num_q_tiles:
         step.q_tiles = buffer[rows_end : rows_end + 2 * layout.num_q_tiles]
         step.num_q_tiles = layout.num_q_tiles
+        step.portions = layout.portions
     return step, buffer[3 * t + b : rows_end]

@@ -99,6 +99,31 @@ def tiles_pay(tokens: int, portions: int, keys: int, heads: int, size: int) -> b
     return tiled < 0.9 * plain
 
 
+def pairs_pay(portions: list, heads: int, kv_heads: int, window: int, longest: int, sms: int) -> bool:
+    """Whether attention of prompt portions (``(cached, new)`` tokens each) is faster with two query tiles a CTA and keys cut
+    into equal shares (attention_prefill_pairs.cu) than with a CTA per tile and head (attention_prefill_tcgen05.cu).
+
+    Two estimates in us from the blocks of 128 keys that the tiles of 128 tokens see, fitted to 1,365 steps timed both ways (1 to
+    48 heads in groups of 1 to 8, heads of 64 and 128, 1 to 32 portions of 2 to 3,000 tokens behind up to 9,000, windows).  A
+    tile to itself takes a block in less time than one of a pair does, so steps whose longest tile takes the time are the
+    first kernel's, and steps with work for all SMs, or with long rows of keys that can be cut, the second one's (us, one /
+    two tiles a CTA: 12 heads, 2,048 tokens 30.7 / 33.5; 28 heads, 2,048 behind 4,000 253 / 150; 12 heads, 130 behind 6,000 76 / 33;
+    28 heads, 64 portions of 2 behind 100 99 / 49; 64 tokens behind 200 12 / 17).  0.9: where the estimates err."""
+    tiles = blocks = most = 0
+    for past, tokens in portions:
+        count, first = -(-tokens // 128), (past + 127) // 128 + 1  # tiles, and the blocks that the first of them sees
+        cap = (window + 253) // 128 + 1 if window else 1 << 30
+        rising = min(count, max(0, cap - first))
+        tiles += count
+        blocks += rising * first + rising * (rising - 1) // 2 + (count - rising) * cap if rising < count else (
+            count * first + count * (count - 1) // 2)
+        most = max(most, min(first + count - 1, cap))
+    units = tiles * heads / 2 if heads // kv_heads % 2 == 0 else 0.8 * tiles * heads
+    one = 6.5 + ((1.43 * most) ** 3 + ((1.43 * blocks + 5.8 * tiles) * heads / sms) ** 3) ** (1 / 3)
+    two = 8.1 + (6.8 if longest > 1024 else 0.0) + math.hypot(2.0 * min(most, 8), (blocks * heads + 7.0 * units) / sms)
+    return two < 0.9 * one
+
+
 class DeviceKernels(KernelSet):
     def __init__(self, dtype: torch.dtype, device: torch.device | str = "cuda:0") -> None:
         if dtype not in _CODE:
@@ -587,18 +612,41 @@ class DeviceKernels(KernelSet):
     def _attention_tcgen05(self, qkv, out, step, kv, num_heads, num_kv_heads, head_dim, window, chunk, scale,
                            keep_first=0, softcap=0.0, sink_ptr=None) -> bool:
         """Prompt portions on the tcgen05 kernel; False when it refuses the page size or an alignment."""
-        code = function("distie_attention_prefill_tcgen05")(
+        args = [
             qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), step.q_tiles.data_ptr(), step.num_q_tiles,
             step.positions.data_ptr(), step.token_seq.data_ptr(), step.seq_seat.data_ptr(),
             kv.block_table.data_ptr(), kv.block_table.shape[-1], kv.k.data_ptr(), kv.v.data_ptr(), qkv.shape[0],
             num_heads, num_kv_heads, head_dim, kv.v.shape[-1], kv.page_size, kv.num_pages, window, chunk, keep_first, float(scale),
-            float(softcap), sink_ptr, self.error_flag.data_ptr(), self._stream(),
-        )
+            float(softcap), sink_ptr,
+        ]
+        kernels = 1
+        if self._in_pairs(step, num_heads, num_kv_heads, window, chunk):
+            floats = function("distie_attention_prefill_pairs_scratch_floats")(step.max_kv_len, kv.v.shape[-1], self.sm_count)
+            scratch = torch.empty(floats, dtype=torch.float32, device=qkv.device) if floats else None  # parts of long portions
+            kernels = 2 if floats else 1
+            code = function("distie_attention_prefill_pairs")(*args, scratch.data_ptr() if floats else None, self.sm_count,
+                                                              self.error_flag.data_ptr(), self._stream())
+        else:
+            code = function("distie_attention_prefill_tcgen05")(*args, self.error_flag.data_ptr(), self._stream())
         if code == -2:
             return False
         check(code, "attention_prefill_tcgen05")
-        self._ran("attention_prefill_tcgen05")
+        self._ran("attention_prefill_tcgen05", kernels)
         return True
+
+    def _in_pairs(self, step, num_heads: int, num_kv_heads: int, window: int, chunk: int) -> bool:
+        if step.max_kv_len <= 2048 and step.num_q_tiles * num_heads < 2 * self.sm_count:
+            return False  # (no step of the 1,365 behind pairs_pay's estimates in this range is sent to the pairs by them)
+        key = ("pairs", num_heads, num_kv_heads, window, chunk)
+        made = step.derived.get(key)
+        if made is None:
+            portions = step.portions
+            if portions is None:  # portions of equal length that end at the longest one's last key
+                count = max(1, step.num_seqs - step.num_decode_tokens)
+                mean = -(-(step.num_tokens - step.num_decode_tokens) // count)
+                portions = [(max(0, step.max_kv_len - mean), mean)] * count
+            made = step.derived[key] = pairs_pay(portions, num_heads, num_kv_heads, window or chunk, step.max_kv_len, self.sm_count)
+        return made
 
     # -- layers with per-request state: layer norm over a pending sum, gates, convolutions, recurrences ---------
     def add_layernorm(self, delta, residual, weight, bias, eps, out, rows_index=None) -> None:

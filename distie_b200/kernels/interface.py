@@ -45,6 +45,7 @@ class StepTensors:
     max_kv_len: int = 0  # bound on the keys any token sees; a captured step uses a fixed bound
     q_tiles: torch.Tensor | None = None  # [n, 2] int32: (first token, rows <= Q_TILE) of each tile of the
     num_q_tiles: int = 0                 # multi-token entries; a tile holds consecutive tokens of one request
+    portions: list | None = None         # (cached tokens, new tokens) of the multi-token entries, where the host knows them
     derived: dict = field(default_factory=dict)  # what a kernel set made of this step once and its layers share
 
 

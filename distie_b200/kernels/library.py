@@ -50,6 +50,10 @@ _SIGNATURES: dict[str, tuple[str, list]] = {
     "distie_attention_prefill_tcgen05": (
         "bf16", [P, I, P, I, P, I, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, I, I, F, F, P, P, P]
     ),
+    "distie_attention_prefill_pairs": (
+        "bf16", [P, I, P, I, P, I, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, I, I, F, F, P, P, I, P, P]
+    ),
+    "distie_attention_prefill_pairs_scratch_floats": ("bf16", [I, I, I]),
     "distie_attention_decode_mma_ragged": (
         "bf16", [P, I, P, I, P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, I, F, F, P, I, I, I, P, P]
     ),
@@ -129,7 +133,7 @@ _SIGNATURES: dict[str, tuple[str, list]] = {
     "distie_gemm_tcgen05_skinny_act": ("bf16", [P, I, P, P, I, I, I, I, I, F, F, I, P, P]),
     "distie_gemm_tcgen05_skinny": ("bf16", [P, I, P, P, P, I, I, I, I, I, I, I, P, P]),
 }
-_RESULT = {"distie_retention_scratch_floats": c_longlong, "distie_recurrence_chunks_scratch_floats": c_longlong,
+_RESULT = {"distie_attention_prefill_pairs_scratch_floats": c_longlong, "distie_retention_scratch_floats": c_longlong, "distie_recurrence_chunks_scratch_floats": c_longlong,
            "distie_exp_gate_scratch_floats": c_longlong, "distie_attention_decode_scratch_floats": c_longlong, "distie_route_plan_words": c_longlong,
            "distie_latent_attention_scratch_floats": c_longlong, "distie_selective_scan_scratch_floats": c_longlong,
            "distie_channel_delta_scratch_floats": c_longlong}

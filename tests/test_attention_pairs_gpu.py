@@ -1,0 +1,110 @@
+"""Attention of prompt portions with two query tiles a CTA and keys cut into shares, against the formulas in float32.
+
+Groups that pair up and groups that do not, tiles without a partner, units cut into pieces and rows of units cut into
+shares, partial tiles, every mask and score option, heads that fill no tile, pages of every size, scores that rise by
+more than the range in which exponentials are taken without a new maximum."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+import ref_kernels as ref
+from test_kernels_gpu import close, filled_cache_for, step_of
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ks():
+    from distie_b200.kernels import make_kernels
+
+    return make_kernels(torch.bfloat16, "cuda:0")
+
+
+def run(ks, monkeypatch, heads, kv_heads, head_dim, value_dim, page, tokens, pasts, window=None, chunk=None, keep_first=0, softcap=0.0,
+        sink=False, scale=None, keys=None, missing=None):
+    from distie_b200.kernels import device
+    from distie_b200.kernels.interface import KvSlot
+
+    monkeypatch.setattr(device, "pairs_pay", lambda *args: True)
+    g = torch.Generator(device="cuda").manual_seed(heads * 31 + head_dim + sum(tokens))
+    kv = filled_cache_for(torch.bfloat16, kv_heads, head_dim, page, [p + n for p, n in zip(pasts, tokens)])
+    values = torch.randn(*kv.k.shape[:3], value_dim, generator=g, device="cuda").to(torch.bfloat16)
+    kv = KvSlot(kv.k, values, kv.block_table, page, kv.num_pages)
+    if keys is not None:
+        keys(kv)
+    step = step_of(tokens, pasts, list(range(len(tokens))))
+    q = torch.randn(step.num_tokens, heads * head_dim, generator=g, device="cuda").to(torch.bfloat16)
+    sinks = torch.randn(heads, generator=g, device="cuda") if sink else None
+    out = torch.full((step.num_tokens, heads * value_dim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    before = ks.kernel_counts.get("attention_prefill_tcgen05", 0)
+    args = (heads, kv_heads, head_dim, window, scale or head_dim**-0.5, chunk, keep_first, softcap, sinks)
+    want = ref.attention(q, step, kv, *args)
+    if missing is not None:
+        missing(kv)
+    ks.attention(q, out, step, kv, *args)
+    ks.check_errors()
+    assert ks.kernel_counts["attention_prefill_tcgen05"] == before + 1
+    close(out, want, torch.bfloat16, f"{heads} heads, {tokens} behind {pasts}")
+
+
+@pytest.mark.parametrize("heads,kv_heads", [(4, 2), (6, 2), (7, 1), (3, 3), (1, 1), (40, 8)])
+@pytest.mark.parametrize("tokens,pasts", [
+    ([2], [0]), ([128], [0]), ([129], [0]), ([257], [3]), ([300, 2, 128, 511], [900, 4000, 0, 1]), ([150], [5000]), ([1, 1, 700], [30, 2000, 1500]),
+])
+def test_units_pieces_and_shares(ks, monkeypatch, heads, kv_heads, tokens, pasts):
+    run(ks, monkeypatch, heads, kv_heads, 128, 128, 16, tokens, pasts)
+
+
+def test_more_tiles_than_lanes_and_units_than_shares(ks, monkeypatch):
+    run(ks, monkeypatch, 6, 2, 64, 64, 16, [2 + 5 * i for i in range(70)], [37 * (i % 9) for i in range(70)])
+    run(ks, monkeypatch, 14, 2, 128, 128, 16, [260] * 9 + [1300], [1000] * 9 + [2100])
+
+
+@pytest.mark.parametrize("head_dim,value_dim,page,window,chunk,keep_first,softcap,sink", [
+    (128, 128, 8, 300, None, 0, 0.0, False), (64, 64, 128, 1000, None, 40, 0.0, True), (128, 128, 32, None, 500, 0, 0.0, False),
+    (96, 96, 16, 64, None, 200, 0.0, False), (128, 64, 16, None, None, 0, 5.0, True), (64, 128, 64, 200, None, 3, 2.5, False),
+    (40, 8, 16, None, 128, 0, 0.0, True), (88, 120, 16, 1, None, 0, 0.0, False),
+])
+@pytest.mark.parametrize("heads,kv_heads", [(6, 3), (5, 1)])
+def test_masks_caps_sinks_and_sizes(ks, monkeypatch, heads, kv_heads, head_dim, value_dim, page, window, chunk, keep_first, softcap, sink):
+    run(ks, monkeypatch, heads, kv_heads, head_dim, value_dim, page, [1, 333, 2, 140], [10, 1700, 900, 0], window, chunk, keep_first, softcap, sink)
+
+
+@pytest.mark.parametrize("kv_heads", [1, 2])
+def test_pages_that_a_window_gave_back_are_not_asked_for(ks, monkeypatch, kv_heads):
+    pasts, window = [2000, 650], 300
+
+    def missing(kv):
+        for seat, past in enumerate(pasts):
+            kv.block_table[seat, : max(0, past - window + 1) // 16] = -1
+
+    run(ks, monkeypatch, 2, kv_heads, 128, 128, 16, [300, 290], pasts, window, missing=missing)
+
+
+@pytest.mark.parametrize("factor,scale", [(1.0, 3.0), (4.0, 2.0)])
+def test_scores_that_leave_the_range(ks, monkeypatch, factor, scale):
+    """Keys grow along the request: a row's scores rise by hundreds in base-2 units, past 2^30 many times over."""
+    def keys(kv):
+        growth = torch.linspace(0.01, factor, kv.block_table.shape[1], device="cuda")
+        for seat in range(kv.block_table.shape[0]):
+            row = kv.block_table[seat]
+            held = row[row >= 0].long()
+            kv.k[held] = (kv.k[held].float() * growth[: held.numel(), None, None, None]).to(torch.bfloat16)
+
+    run(ks, monkeypatch, 4, 2, 128, 128, 16, [200, 150], [1800, 300], scale=scale, keys=keys)
+
+
+def test_a_missing_page_sets_the_error_word(ks, monkeypatch):
+    from distie_b200.kernels import device
+    from distie_b200.kernels.library import KernelError
+
+    monkeypatch.setattr(device, "pairs_pay", lambda *args: True)
+    kv = filled_cache_for(torch.bfloat16, 2, 128, 16, [1500])
+    kv.block_table[0, 40] = -1
+    step = step_of([200], [1300], [0])
+    q = torch.randn(200, 4 * 128, device="cuda").to(torch.bfloat16)
+    ks.attention(q, torch.empty_like(q), step, kv, 4, 2, 128, None, 128**-0.5)
+    with pytest.raises(KernelError):
+        ks.check_errors()

@@ -7,7 +7,7 @@ from __future__ import annotations
 
 import pytest
 
-from distie_b200.kernels.device import chunks_pay, tiles_pay
+from distie_b200.kernels.device import chunks_pay, pairs_pay, tiles_pay
 
 
 @pytest.mark.parametrize("rule,key,value,heads,portions,tokens,walk,chunks", [
@@ -48,3 +48,19 @@ def test_recurrences_run_in_chunks_where_that_is_faster(rule, key, value, heads,
 ])
 def test_float32_attention_runs_in_tiles_where_that_is_faster(heads, size, portions, tokens, past, plain, tiles):
     assert tiles_pay(portions * tokens, portions, tokens + past, heads, size) == (tiles < plain)
+
+
+@pytest.mark.parametrize("heads,kv_heads,window,portions,one,two", [
+    # heads, those of keys, window, (cached, new) tokens of the portions, us with one and with two tiles a CTA
+    (12, 2, 0, [(0, 130)], 10.3, 12.5),
+    (12, 2, 0, [(6000, 130)], 76.3, 33.0),
+    (12, 2, 0, [(0, 1024)], 18.4, 22.9),
+    (12, 2, 0, [(9000, 1000)], 123.1, 72.2),
+    (28, 4, 0, [(4000, 2048)], 252.9, 149.8),
+    (28, 4, 0, [(100, 2)] * 64, 99.2, 48.6),
+    (40, 8, 0, [(200, 64)], 12.6, 17.4),
+    (7, 1, 0, [(0, 777)], 17.2, 21.5),
+    (8, 8, 0, [(0, 128)] * 16, 7.8, 10.8),
+])
+def test_prompt_attention_takes_two_tiles_a_cta_where_that_is_faster(heads, kv_heads, window, portions, one, two):
+    assert pairs_pay(portions, heads, kv_heads, window, max(p + n for p, n in portions), 148) == (two < one)

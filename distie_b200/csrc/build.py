@@ -47,6 +47,8 @@ CUDA_UNITS: dict[str, list[str]] = {
     # bfloat16 serving only: tensor-core attention for prompts, weight-streaming products for decoding
     "bf16": ["attention_prefill.cu", "attention_decode_mma.cu", "gemm_tcgen05.cu", "attention_prefill_tcgen05.cu",
              "attention_prefill_pairs.cu"],
+    # float32 products of many rows
+    "float32": ["gemm_float32.cu"],
     # models with layer norms, gated heads, short convolutions or linear recurrences (both dtypes)
     "state": ["recurrent.cu", "recurrence_chunks.cu", "retention.cu"],
     # models with recurrences whose decay varies by channel (both dtypes); a unit of its own because it takes minutes

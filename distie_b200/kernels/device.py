@@ -7,7 +7,8 @@ element type of activations, weights and cache, and in the matrix products:
   library (cuBLAS through ``torch.mm``), as the reference's engine does for every
   product (worker/src/inference/qwen2/model.py:216-236); skinny and fused
   products use this package's own kernels where they are registered.
-* float32: ``torch.mm`` with TF32 switched off, i.e. FMA-only float32 products;
+* float32: many rows on the tensor cores, every float32 number as three bfloat16 ones, nearer to 64-bit values than
+  FMA products are (gemm_float32.cu); few rows through ``torch.mm`` with TF32 switched off, i.e. FMA-only products;
   accurate ``expf``/``sincosf``/``rsqrtf`` in every kernel.
 
 There is no CPU path here and no fallback: a missing library raises.
@@ -97,6 +98,20 @@ def tiles_pay(tokens: int, portions: int, keys: int, heads: int, size: int) -> b
     plain = 3.0 + (0.6 + 0.3 * size / 128) * -(-keys // 4) * max(1.0, tokens * heads / 710) ** 0.81 + 0.113 * tokens * heads / 148
     tiled = 2.4 + (2.2 + 5.2 * wide) * -(-keys // 64) * max(1.0, blocks / 296) + 5.2 * wide * blocks / 148
     return tiled < 0.9 * plain
+
+
+def wide_pays(m: int, n: int, k: int, sms: int) -> bool:
+    """Whether the float32 product ``[m, k] x [n, k]^T`` is faster on the tensor cores (gemm_float32.cu) than in the library.
+
+    Two estimates in us: the planes of both operands and whole waves of 128 x 128 tiles, fitted to 178 products timed both ways (40
+    to 3,000 rows, 64 to 20,000 columns, K of 64 to 9,600); and the library at 50 TFLOP/s, which it reaches where tiles are
+    many, so that none of the 178 is sent to the slower one (tensor cores / library, us: 777 x 2,048 x 1,536 39 / 112, 2,048 x
+    2,048 x 1,536 74 / 247, 1,024 x 8,960 x 1,536 158 / 514, 128 x 2,048 x 1,536 36 / 34).  The planes take 6 bytes a number of both
+    operands while the product runs: up to as much as the states between chunks may."""
+    if 6 * (m + n) * k > _CHUNK_BYTES:
+        return False
+    waves = -(-(-(-m // 128) * -(-n // 128)) // sms)
+    return 6.6 + 2.04e-6 * (m + n) * k + 0.0194 * waves * k < 0.95 * (6.0 + m * n * k * 4e-8)
 
 
 def pairs_pay(portions: list, heads: int, kv_heads: int, window: int, longest: int, sms: int) -> bool:
@@ -243,7 +258,9 @@ class DeviceKernels(KernelSet):
         if weight.dtype == torch.float32:
             # float32 engine, or a matrix the checkpoint stores in 32-bit: a true float32 product.
             x32 = x if x.dtype == torch.float32 else x.float()
-            y = torch.addmm(bias, x32, weight.t()) if bias is not None else torch.mm(x32, weight.t())
+            y = self._float32_product(x32, weight, bias)
+            if y is None:
+                y = torch.addmm(bias, x32, weight.t()) if bias is not None else torch.mm(x32, weight.t())
             return y if out_dtype == torch.float32 else self._bias_cast(y, None, out_dtype)
         if self._skinny(x, weight):
             out = torch.empty((x.shape[0], weight.shape[0]), dtype=out_dtype, device=x.device)
@@ -259,6 +276,25 @@ class DeviceKernels(KernelSet):
         if out_dtype == torch.float32:
             return y32 if bias is None else y32.add_(bias)
         return self._bias_cast(y32, bias, out_dtype)
+
+    def _float32_product(self, x, weight, bias):
+        """Many rows on the tensor cores, three bfloat16 numbers for every float32 one (gemm_float32.cu); None where the
+        library is faster, or for sizes that the kernel does not take."""
+        m, n, k = x.shape[0], weight.shape[0], weight.shape[1]
+        if not wide_pays(m, n, k, self.sm_count) or x.stride(1) != 1 or not weight.is_contiguous() or (bias is not None and (
+                bias.dtype != torch.float32 or not bias.is_contiguous())):
+            return None
+        out = torch.empty((m, n), dtype=torch.float32, device=x.device)
+        scratch = torch.empty(function("distie_gemm_float32_scratch_floats")(m, n, k), dtype=torch.float32, device=x.device)
+        code = function("distie_gemm_float32")(
+            x.data_ptr(), x.stride(0), weight.data_ptr(), bias.data_ptr() if bias is not None else None, out.data_ptr(), n, m, n, k,
+            scratch.data_ptr(), self.error_flag.data_ptr(), self._stream(),
+        )
+        if code == -2:
+            return None
+        check(code, "gemm_float32")
+        self._ran("gemm_float32", 2)
+        return out
 
     def _tensor_core(self, x, weight) -> bool:
         """Products of more rows than the weight-streaming kernel takes: the tcgen05 kernel."""

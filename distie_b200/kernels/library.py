@@ -78,6 +78,8 @@ _SIGNATURES: dict[str, tuple[str, list]] = {
     "distie_recurrence_chunks": (
         "state", [I, P, I, P, I, P, I, P, I, P, I, I, L, P, P, P, P, P, I, P, P, I, P, P, I, I, I, I, I, F, P, P, P]
     ),
+    "distie_gemm_float32_scratch_floats": ("float32", [I, I, I]),
+    "distie_gemm_float32": ("float32", [P, I, P, P, P, I, I, I, I, P, P, P]),
     "distie_activation": ("state", [P, I, I, L, P, I, I, I, F, I, I, P]),
     "distie_retention_scratch_floats": ("state", [I, I, I, I]),
     "distie_retention_chunks": (
@@ -133,7 +135,7 @@ _SIGNATURES: dict[str, tuple[str, list]] = {
     "distie_gemm_tcgen05_skinny_act": ("bf16", [P, I, P, P, I, I, I, I, I, F, F, I, P, P]),
     "distie_gemm_tcgen05_skinny": ("bf16", [P, I, P, P, P, I, I, I, I, I, I, I, P, P]),
 }
-_RESULT = {"distie_attention_prefill_pairs_scratch_floats": c_longlong, "distie_retention_scratch_floats": c_longlong, "distie_recurrence_chunks_scratch_floats": c_longlong,
+_RESULT = {"distie_gemm_float32_scratch_floats": c_longlong, "distie_attention_prefill_pairs_scratch_floats": c_longlong, "distie_retention_scratch_floats": c_longlong, "distie_recurrence_chunks_scratch_floats": c_longlong,
            "distie_exp_gate_scratch_floats": c_longlong, "distie_attention_decode_scratch_floats": c_longlong, "distie_route_plan_words": c_longlong,
            "distie_latent_attention_scratch_floats": c_longlong, "distie_selective_scan_scratch_floats": c_longlong,
            "distie_channel_delta_scratch_floats": c_longlong}

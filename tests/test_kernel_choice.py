@@ -7,7 +7,7 @@ from __future__ import annotations
 
 import pytest
 
-from distie_b200.kernels.device import chunks_pay, pairs_pay, tiles_pay
+from distie_b200.kernels.device import chunks_pay, pairs_pay, tiles_pay, wide_pays
 
 
 @pytest.mark.parametrize("rule,key,value,heads,portions,tokens,walk,chunks", [
@@ -64,3 +64,11 @@ def test_float32_attention_runs_in_tiles_where_that_is_faster(heads, size, porti
 ])
 def test_prompt_attention_takes_two_tiles_a_cta_where_that_is_faster(heads, kv_heads, window, portions, one, two):
     assert pairs_pay(portions, heads, kv_heads, window, max(p + n for p, n in portions), 148) == (two < one)
+
+
+@pytest.mark.parametrize("m,n,k,wide,library", [
+    (777, 2048, 1536, 39.1, 111.5), (128, 512, 512, 26.0, 13.1), (2048, 8960, 1536, 390.0, 964.6), (64, 2048, 1536, 36.0, 29.8),
+    (512, 512, 512, 17.0, 15.2), (1024, 1536, 8960, 220.0, 596.0), (32, 8960, 1536, 76.8, 33.5),
+])
+def test_float32_products_run_on_the_tensor_cores_where_that_is_faster(m, n, k, wide, library):
+    assert wide_pays(m, n, k, 148) == (wide < library)

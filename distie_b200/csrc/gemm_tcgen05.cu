@@ -786,6 +786,152 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 }
 
 // ---------------------------------------------------------------------------------------------------------------
+// Pairs of CTAs over groups of rows (see gemm_tcgen05_grouped_kernel): the list's tiles have up to 256 rows, 128 a CTA.  The
+// grouped product is bound by what an SM pulls out of L2, 96 bytes a cycle of MMAs in tiles of 128 rows, 64 here.
+// ---------------------------------------------------------------------------------------------------------------
+template <int STAGES, int EPI>
+__global__ void __launch_bounds__(kGemmWideThreads, 1)
+gemm_tcgen05_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                                 void* __restrict__ out, int ldo, int N, int K, int inter, int num_tiles, const GroupedTiles tiles,
+                                 float limit, HiddenAct act, int* __restrict__ error) {
+  constexpr int BN = 256;
+  extern __shared__ unsigned char raw[];
+  auto& sm = *reinterpret_cast<PairShared<BN, STAGES, 1>*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
+  constexpr uint32_t TMEM_COLS = 512;   // two accumulators, the second at column 256
+  constexpr uint32_t ACC_STRIDE = 256;
+  constexpr uint32_t STAGE_BYTES_PAIR = 2 * (kGemmBM + BN / 2) * kGemmBK * 2;
+  constexpr int PER_TILE = EPI == GEMM_EPI_SWIGLU ? BN / 2 : BN;  // output columns per tile
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k_blocks = (K + kGemmBK - 1) / kGemmBK;
+  const uint32_t rank = cluster_cta_rank();       // 0: issues the MMAs
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  if (threadIdx.x == 64) {
+    prefetch_tensor_map(&map_a);
+    prefetch_tensor_map(&map_b);
+  }
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&sm.full[s], 1);
+      mbar_init(&sm.empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&sm.accum_full[b], 1);
+      mbar_init(&sm.accum_empty[b], 16);  // one arrival per epilogue warp of the pair
+    }
+    sm.failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)),
+                 "r"(TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  cluster_barrier();  // both CTAs' barriers are initialised and tensor memory is allocated
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = sm.tmem_base;
+  grid_dependency_release();
+  grid_dependency_wait();  // the list of tiles comes from a kernel before this one
+  const int m_tiles = min(*tiles.num_m_tiles, tiles.max_m_tiles);
+
+  if (warp == 0) {
+    // ---- producer (both CTAs) -------------------------------------------------------------------------------
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
+        const int mt = tile % tiles.max_m_tiles;
+        if (mt >= m_tiles) continue;
+        const int m0 = tiles.first[mt] + (int)rank * kGemmBM, column = (tile / tiles.max_m_tiles) * PER_TILE;
+        // Rows of W this CTA stages: with SwiGLU the first CTA takes the gate rows, the second the up rows.
+        const int w0 = tiles.group[mt] * tiles.w_rows + column + (EPI == GEMM_EPI_SWIGLU ? (int)rank * inter : (int)rank * (BN / 2));
+        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait_unless(&sm.empty[s], ((it / STAGES) & 1) ^ 1, &sm.failed)) { ok = false; break; }
+          if (rank == 0) mbar_expect_tx(&sm.full[s], STAGE_BYTES_PAIR);
+          const uint32_t full_addr = cluster_address(&sm.full[s], 0);
+          tma_load_2d_pair(sm.b[s][0], &map_b, full_addr, kb * kGemmBK, w0);
+          tma_load_2d_pair(sm.a[s][0], &map_a, full_addr, kb * kGemmBK, m0);
+        }
+      }
+      if (!ok) {
+        atomicExch(&sm.failed, 1u);
+        // Copies already issued still land in shared memory: the first CTA, whose barriers count them,
+        // gives them a bounded time before the pair leaves.
+        if (rank == 0)
+          for (uint32_t back = (it > (uint32_t)STAGES ? it - STAGES : 0); back < it; ++back)
+            mbar_wait(&sm.full[back % STAGES], (back / STAGES) & 1);
+      }
+    }
+  } else if (warp == 1) {
+    // ---- MMA issuer (first CTA only) --------------------------------------------------------------------------
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc = instr_desc_pair(BN);
+      uint32_t it = 0, round = 0;
+      bool ok = true;
+      for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
+        if (tile % tiles.max_m_tiles >= m_tiles) continue;
+        const uint32_t buffer = round & 1;
+        if (!mbar_wait_unless(&sm.accum_empty[buffer], ((round >> 1) & 1) ^ 1, &sm.failed)) { ok = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = tmem + buffer * ACC_STRIDE;
+        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait_unless(&sm.full[s], (it / STAGES) & 1, &sm.failed)) { ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint64_t a_desc = smem_desc(sm.a[s][0]), b_desc = smem_desc(sm.b[s][0]);
+#pragma unroll
+          for (int k = 0; k < kGemmBK / 16; ++k)
+            umma_bf16_pair(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(&sm.empty[s], 3);
+        }
+        if (ok) umma_commit_pair(&sm.accum_full[buffer], 3);
+        ++round;
+      }
+      if (!ok) atomicExch(&sm.failed, 1u);
+    }
+  } else {
+    // ---- epilogue (both CTAs, each its own 128 rows; two warps per quarter of the rows, half the columns each) --
+    const int quadrant = warp & 3, part = (warp - 2) >> 2;
+    unsigned char* behind = reinterpret_cast<unsigned char*>(&sm) + ((sizeof(sm) + 15) & ~size_t(15));  // (the float32 epilogue's)
+    unsigned char* epilogue_stage = behind + (warp - 2) * kEpilogueStageBytes;
+    uint32_t round = 0;
+    for (int tile = pair; tile < num_tiles; tile += pairs) {
+      const int mt = tile % tiles.max_m_tiles;
+      if (mt >= m_tiles) continue;
+      const uint32_t buffer = round & 1;
+      const int end = tiles.first[mt] + tiles.rows[mt], m0 = tiles.first[mt] + (int)rank * kGemmBM;
+      const int n0 = (tile / tiles.max_m_tiles) * PER_TILE;
+      const bool ready = __all_sync(0xffffffffu, mbar_wait_unless(&sm.accum_full[buffer], (round >> 1) & 1, &sm.failed));
+      if (!ready) { atomicExch(&sm.failed, 1u); break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t lane_base = tmem + buffer * ACC_STRIDE + ((uint32_t)(quadrant * 32) << 16);
+      // (rows of the box past the group's own are not stored)
+      if (m0 + quadrant * 32 < end)
+        store_accumulator<BN, EPI>(lane_base, m0 + quadrant * 32, lane, n0, out, ldo, end, N, inter, part, epilogue_stage, limit, act);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster_relaxed(cluster_address(&sm.accum_empty[buffer], 0));
+      ++round;
+    }
+  }
+
+  // Neither CTA may leave while the other can still reach its shared memory, barriers or tensor memory.
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (sm.failed && threadIdx.x == 0) {
+    // Tell the other CTA, so that its waits end at once, and give copies in flight time to land.
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_address(&sm.failed, rank ^ 1)), "r"(1u) : "memory");
+    __nanosleep(20000);
+  }
+  cluster_barrier_exit();
+  if (warp == 1) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+  }
+  if (threadIdx.x == 0 && sm.failed && error) atomicExch(error, 6);
+}
+
+// ---------------------------------------------------------------------------------------------------------------
 // The same machinery turned around for few rows of x (decoding): the weights are the 128-row operand and
 // stream through a deep ring of TMA stages (16 KB each), the rows of x are the narrow operand
 // (N = 16, 32 or 64), and the accumulator is D[weight row, row of x].  A product like this is bound by
@@ -1184,6 +1330,42 @@ extern "C" int distie_gemm_tcgen05_split(const void* x, int ldx, const void* w, 
                     : launch_gemm_pair<128, 8, 1, GEMM_EPI_F32>(map_a, map_b, out, N, M, N, K, 0, sm_count, error, stream);
 }
 
+template <int EPI>
+static int launch_grouped_pairs(const CUtensorMap& map_a, const CUtensorMap& map_b, void* out, int ldo, int N, int K, int inter,
+                                const GroupedTiles& tiles, float limit, HiddenAct act, int sm_count, int* error, cudaStream_t stream) {
+  constexpr int STAGES = 6;
+  const size_t shared = sizeof(PairShared<256, STAGES, 1>) + 1024 + (EPI == GEMM_EPI_F32 ? 16 + 8 * kEpilogueStageBytes : 0);
+  static_assert(sizeof(PairShared<256, STAGES, 1>) + 1024 + 16 + 8 * kEpilogueStageBytes <= 232448, "shared memory of a CTA");
+  static int resident_pairs = 0;  // pairs that can run at the same time (an SM left over in a GPC hosts none)
+  if (resident_pairs == 0) {
+    cudaError_t err = cudaFuncSetAttribute(gemm_tcgen05_grouped_pair_kernel<STAGES, EPI>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+    if (err != cudaSuccess) return (int)err;
+    cudaLaunchConfig_t probe = {};
+    probe.gridDim = dim3(2 * (sm_count / 2));
+    probe.blockDim = dim3(kGemmWideThreads);
+    probe.dynamicSmemBytes = shared;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeClusterDimension;
+    attribute[0].val.clusterDim.x = 2;
+    attribute[0].val.clusterDim.y = 1;
+    attribute[0].val.clusterDim.z = 1;
+    probe.attrs = attribute;
+    probe.numAttrs = 1;
+    int most = 0;
+    err = cudaOccupancyMaxActiveClusters(&most, gemm_tcgen05_grouped_pair_kernel<STAGES, EPI>, &probe);
+    if (err != cudaSuccess) return (int)err;
+    if (most < 1) return DISTIE_ERR_UNSUPPORTED;
+    resident_pairs = most;
+  }
+  const int per_tile = EPI == GEMM_EPI_SWIGLU ? 128 : 256, columns = EPI == GEMM_EPI_SWIGLU ? inter : N;
+  const int num_tiles = tiles.max_m_tiles * ((columns + per_tile - 1) / per_tile), pairs = min(num_tiles, min(resident_pairs, sm_count / 2));
+  const cudaError_t err = launch_dependent_cluster(64, dim3(2, 1, 1), gemm_tcgen05_grouped_pair_kernel<STAGES, EPI>, dim3(2 * pairs),
+                                                   dim3(kGemmWideThreads), shared, stream, map_a, map_b, out, ldo, N, K, inter, num_tiles,
+                                                   tiles, limit, act, error);
+  return err == cudaSuccess ? 0 : (int)err;
+}
+
 // The grouped product (see gemm_tcgen05_grouped_kernel): a[rows_a, K] sorted by group, w[groups * w_rows, K]; the tile
 // list lives on the device.  epi 2: w_rows = 2 * inter and out[rows_a, inter] bfloat16 = silu(a Wg^T) * (a Wu^T), or with
 // limit > 0 its capped form g' sigmoid(1.702 g') (u' + 1), g' = min(g, limit), u' = clamp(u, -limit, limit);
@@ -1192,8 +1374,9 @@ extern "C" int distie_gemm_tcgen05_split(const void* x, int ldx, const void* w, 
 extern "C" int distie_gemm_tcgen05_grouped(const void* a, int lda, int rows_a, const void* w, int groups, int w_rows,
                                            void* out, int ldo, int N, int K, int epi, float limit, int kind, float act_a,
                                            float act_b, const int* num_m_tiles, const int* tile_group, const int* tile_first,
-                                           const int* tile_rows, int max_m_tiles, int sm_count, int* error,
+                                           const int* tile_rows, int max_m_tiles, int tile, int sm_count, int* error,
                                            cudaStream_t stream) {
+  if (tile != kGemmBM && tile != 2 * kGemmBM) return DISTIE_ERR_ARG;
   if (rows_a <= 0 || max_m_tiles <= 0) return 0;
   if (N < 1 || K < 8 || (K & 7) || (lda & 7) || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || groups < 1 || w_rows < 1)
     return DISTIE_ERR_UNSUPPORTED;
@@ -1204,6 +1387,16 @@ extern "C" int distie_gemm_tcgen05_grouped(const void* a, int lda, int rows_a, c
   if (status != 0) return status;
   const GroupedTiles tiles{num_m_tiles, tile_group, tile_first, tile_rows, max_m_tiles, w_rows};
   const HiddenAct act{kind, act_a, act_b};
+  if (tile == 2 * kGemmBM) {
+    if (w_rows != (epi == GEMM_EPI_SWIGLU ? 2 * N : N) || (epi == GEMM_EPI_ACT && (kind < DISTIE_ACT_RELU2 || kind > DISTIE_ACT_XIELU)))
+      return DISTIE_ERR_ARG;
+    if ((status = make_map(&map_b, w, groups * w_rows, K, K, 128)) != 0) return status;
+    if (epi == GEMM_EPI_ACT) return launch_grouped_pairs<GEMM_EPI_ACT>(map_a, map_b, out, ldo, N, K, 0, tiles, 0.f, act, sm_count, error, stream);
+    if (epi == GEMM_EPI_SWIGLU)
+      return launch_grouped_pairs<GEMM_EPI_SWIGLU>(map_a, map_b, out, ldo, 2 * N, K, N, tiles, limit, act, sm_count, error, stream);
+    if (epi == GEMM_EPI_F32) return launch_grouped_pairs<GEMM_EPI_F32>(map_a, map_b, out, ldo, N, K, 0, tiles, 0.f, act, sm_count, error, stream);
+    return DISTIE_ERR_ARG;
+  }
   if (epi == GEMM_EPI_ACT) {
     if (w_rows != N || kind < DISTIE_ACT_RELU2 || kind > DISTIE_ACT_XIELU) return DISTIE_ERR_ARG;
     if ((status = make_map(&map_b, w, groups * w_rows, K, K, 256)) != 0) return status;

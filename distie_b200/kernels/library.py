@@ -106,7 +106,7 @@ _SIGNATURES: dict[str, tuple[str, list]] = {
     "distie_route_plan": ("routed", [P, P, I, I, I, I, P, P, I, P]),
     "distie_routed_gather": ("routed", [P, I, P, I, I, I, P, I, I, I, P]),
     "distie_routed_scatter": ("routed", [P, P, I, I, I, P, I, I, P]),
-    "distie_gemm_tcgen05_grouped": ("bf16", [P, I, I, P, I, I, P, I, I, I, I, F, I, F, F, P, P, P, P, I, I, P, P]),
+    "distie_gemm_tcgen05_grouped": ("bf16", [P, I, I, P, I, I, P, I, I, I, I, F, I, F, F, P, P, P, P, I, I, I, P, P]),
     "distie_routed_swiglu": ("routed", [P, I, P, P, P, P, P, P, P, I, I, I, I, I, I, F, I, I, P, P]),
     "distie_routed_act": ("routed", [P, I, P, P, P, P, P, P, P, I, I, I, I, I, I, F, F, I, P, P]),
     "distie_latent_kv_write": (

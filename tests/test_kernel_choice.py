@@ -7,7 +7,7 @@ from __future__ import annotations
 
 import pytest
 
-from distie_b200.kernels.device import chunks_pay, pairs_pay, tiles_pay, wide_pays
+from distie_b200.kernels.device import chunks_pay, grouped_tile, pairs_pay, tiles_pay, wide_pays
 
 
 @pytest.mark.parametrize("rule,key,value,heads,portions,tokens,walk,chunks", [
@@ -72,3 +72,8 @@ def test_prompt_attention_takes_two_tiles_a_cta_where_that_is_faster(heads, kv_h
 ])
 def test_float32_products_run_on_the_tensor_cores_where_that_is_faster(m, n, k, wide, library):
     assert wide_pays(m, n, k, 148) == (wide < library)
+
+
+@pytest.mark.parametrize("rows,tile", [(12, 128), (75, 128), (112, 128), (131, 128), (169, 256), (188, 256), (394, 256), (562, 128), (750, 256)])
+def test_routed_products_take_the_tile_that_is_not_slower(rows, tile):
+    assert grouped_tile(16 * rows, 16) == tile

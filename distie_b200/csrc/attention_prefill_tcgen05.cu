@@ -1,4 +1,6 @@
-// Attention of prompt portions over the paged cache on the 5th-generation tensor cores, bfloat16.
+// Attention of prompt portions over the paged cache on the 5th-generation tensor cores, bfloat16, a CTA per tile and head: steps
+// whose longest tile takes the time (attention_prefill_pairs.cu takes those with work for the whole machine; pairs_pay in
+// kernels/device.py), and attention through a latent.
 //
 // A CTA takes one tile of up to 128 consecutive query tokens of a request and one query head, and walks
 // the keys the tile may see in blocks of 128:

@@ -96,6 +96,39 @@ def test_scores_that_leave_the_range(ks, monkeypatch, factor, scale):
     run(ks, monkeypatch, 4, 2, 128, 128, 16, [200, 150], [1800, 300], scale=scale, keys=keys)
 
 
+@pytest.mark.parametrize("past", [700, 1500])  # a tile by itself, and one whose keys are cut into pieces
+@pytest.mark.parametrize("low,high", [(15.0, 22.0), (34.0, 60.0)])  # base-2 units: without and with a new maximum
+def test_weights_above_the_maximum_in_use_count_as_they_are_rounded(ks, monkeypatch, past, low, high):
+    """Sixteen keys' scores lie `low` to `high` base-2 units above all before them; their weights, rounded to bfloat16, have to
+    count in the row's sum as they count in the product.  An output is then off along its own direction by no more than its
+    own rounding (2^-9 at most, 1.1e-3 in the root mean square, of each of 128 elements whose squares weigh as normal numbers' do:
+    1.1e-3 (3 / 128)^1/2 = 1.7e-4) and what the other keys' share of 1500 / 2^19 leaves; with weights summed before they are
+    rounded, by up to 2^-9 at once."""
+    from distie_b200.kernels import device
+
+    monkeypatch.setattr(device.DeviceKernels, "_in_pairs", lambda *args: True)
+    g = torch.Generator(device="cuda").manual_seed(past)
+    heads, tokens, at, scale = 4, 200, 32, 128**-0.5  # (keys 512 to 527)
+    kv = filled_cache_for(torch.bfloat16, 2, 128, 16, [past + tokens])
+    kv.k.zero_()
+    kv.k[int(kv.block_table[0, at]), :, :, 0] = 16.0
+    step = step_of([tokens], [past], [0])
+    q = torch.zeros(tokens, heads, 128, device="cuda")
+    q[..., 0] = torch.empty(tokens, heads, device="cuda").uniform_(low, high, generator=g) * 0.6931 / (16 * scale)
+    q = q.to(torch.bfloat16)
+    out = torch.empty(tokens, heads * 128, dtype=torch.bfloat16, device="cuda")
+    ks.attention(q.reshape(tokens, -1), out, step, kv, heads, 2, 128, None, scale)
+    ks.check_errors()
+    keys = torch.arange(past + tokens, device="cuda")
+    pages = kv.block_table[0, keys // 16].long()
+    k, v = (c[pages, :, keys % 16].double().repeat_interleave(heads // 2, dim=1) for c in (kv.k, kv.v))
+    scores = torch.einsum("thd,nhd->thn", q.double(), k) * scale
+    scores.masked_fill_(keys[None, None] > step.positions.long()[:, None, None], float("-inf"))
+    want = torch.einsum("thn,nhd->thd", scores.softmax(-1), v)
+    along = (out.double().reshape_as(want) * want).sum(-1) / (want * want).sum(-1) - 1
+    assert float(along.square().mean().sqrt()) < 3e-4
+
+
 def test_a_missing_page_sets_the_error_word(ks, monkeypatch):
     from distie_b200.kernels import device
     from distie_b200.kernels.library import KernelError

@@ -293,9 +293,14 @@ class DeviceKernels(KernelSet):
     def _float32_product(self, x, weight, bias):
         """Many rows on the tensor cores, three bfloat16 numbers for every float32 one (gemm_float32.cu); None where the
         library is faster, or for sizes that the kernel does not take."""
+        if x.dim() != 2 or weight.dim() != 2 or x.shape[1] != weight.shape[1] or (bias is not None and bias.shape != weight.shape[:1]):
+            return None  # (the library's to refuse, or to take: a bias of another shape that it spreads)
         m, n, k = x.shape[0], weight.shape[0], weight.shape[1]
+        operands = (x, weight) if bias is None else (x, weight, bias)
         if not wide_pays(m, n, k, self.sm_count) or x.stride(1) != 1 or not weight.is_contiguous() or (bias is not None and (
                 bias.dtype != torch.float32 or not bias.is_contiguous())):
+            return None
+        if any(t.device != self.error_flag.device or (t.requires_grad and torch.is_grad_enabled()) for t in operands):
             return None
         out = torch.empty((m, n), dtype=torch.float32, device=x.device)
         scratch = torch.empty(function("distie_gemm_float32_scratch_floats")(m, n, k), dtype=torch.float32, device=x.device)

@@ -6,7 +6,9 @@ quarter and more apart."""
 from __future__ import annotations
 
 import pytest
+import torch
 
+from distie_b200.kernels import device
 from distie_b200.kernels.device import chunks_pay, grouped_tile, pairs_pay, tiles_pay, wide_pays
 
 
@@ -77,3 +79,30 @@ def test_float32_products_run_on_the_tensor_cores_where_that_is_faster(m, n, k, 
 @pytest.mark.parametrize("rows,tile", [(12, 128), (75, 128), (112, 128), (131, 128), (169, 256), (188, 256), (394, 256), (562, 128), (750, 256)])
 def test_routed_products_take_the_tile_that_is_not_slower(rows, tile):
     assert grouped_tile(16 * rows, 16) == tile
+
+
+def test_float32_products_that_the_library_refuses_or_spreads_stay_with_it(monkeypatch):
+    """Operands that do not fit one another never reach the kernel, which takes its sizes from the weight alone."""
+    entered = []
+    monkeypatch.setattr(device, "wide_pays", lambda *args: True)
+    monkeypatch.setattr(device, "function", lambda name: lambda *args: entered.append(name) or 0)
+    ks = device.DeviceKernels.__new__(device.DeviceKernels)
+    ks.dtype, ks.sm_count, ks.error_flag, ks.launches, ks.kernel_counts = torch.float32, 148, torch.zeros(1, dtype=torch.int32), 0, {}
+    ks._stream = lambda: 0
+    x, w = torch.ones(200, 64), torch.ones(128, 64)
+    ks.linear(x, w, torch.ones(128))
+    assert entered and ks.kernel_counts == {"gemm_float32": 1}
+    entered.clear()
+    for wrong in (torch.ones(200, 56), torch.ones(200, 72), torch.ones(64), torch.ones(1, 200, 64)):
+        with pytest.raises(RuntimeError):
+            ks.linear(wrong, w)
+    for bias in (torch.ones(127), torch.ones(129), torch.ones(200, 127)):
+        with pytest.raises(RuntimeError):
+            ks.linear(x, w, bias)
+    with pytest.raises(RuntimeError):
+        ks.linear(x, torch.ones(128, 64, 1))
+    for bias in (torch.ones(1), torch.ones(1, 128), torch.ones(200, 128), torch.ones(200, 1)):
+        assert torch.equal(ks.linear(x, w, bias), torch.full((200, 128), 65.0))
+    grown = torch.ones(128, 64, requires_grad=True)
+    ks.linear(x, grown).sum().backward()
+    assert torch.equal(grown.grad, torch.full((128, 64), 200.0)) and not entered

@@ -250,8 +250,8 @@ __device__ __forceinline__ void share_out(const PairArgs& a, int2* plan, int cta
     // Equal shares where whole units leave CTAs with much less than others (112 units of up to 33 blocks: 24 against 15).
     if (a.partial != nullptr && low > kMinPiece && 4ll * (low + kUnitCost) * ctas > 5 * all + 8ll * ctas) few = false;
   }
-  // What a unit of n blocks counts for: its pieces, or its blocks and kUnitCost.
-  auto weight = [&](int n) { return few ? (n + low - 1) / low : n + kUnitCost; };
+  // What a unit of n blocks counts for: its pieces, or its blocks and kUnitCost.  (Tiles that lead no unit have none of 0 blocks.)
+  auto weight = [&](int n) { return few ? max(1, (n + low - 1) / low) : n + kUnitCost; };
   start.tile = end.tile = a.num_tiles;
   start.unit = start.block = end.unit = end.block = 0;
 #pragma unroll 1

@@ -882,14 +882,14 @@ __global__ void __launch_bounds__(256) merge_pairs_kernel(const __grid_constant_
   if (__ldcg(header) == 0 || half >= __ldcg(header + 1)) return;
   const int t0 = __ldcg(header + 2 + half), rows = __ldcg(header + 4 + half), head = __ldcg(header + 6 + half);
   if (row0 >= rows) return;
-  int parts = 1;
-  for (int base = cta + 1; base < ctas; base += 32) {
+  int parts = 0;
+  for (int base = cta + 1; base < ctas && parts == 0; base += 32) {
     const unsigned ending = __ballot_sync(0xffffffffu, base + lane < ctas && __ldcg(a.headers + 2 * (base + lane) * kPairHeader) == 3);
-    if (ending) {
-      parts += __ffs(ending);
-      break;
-    }
-    parts += 32;
+    if (ending) parts = base - cta + __ffs(ending);
+  }
+  if (parts == 0) {  // (every unit that a CTA begins is ended by one behind it: a plan or a header went wrong)
+    if (threadIdx.x == 0 && a.error) atomicCAS(a.error, 0, 6);
+    return;
   }
   auto part_at = [&](int i) {
     return a.partial + (size_t)(2 * (i == 0 ? 2 * cta + 1 : 2 * (cta + i)) + half) * (kPairRows * (DV + 2));

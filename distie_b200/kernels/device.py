@@ -673,8 +673,8 @@ class DeviceKernels(KernelSet):
             num_heads, num_kv_heads, head_dim, kv.v.shape[-1], kv.page_size, kv.num_pages, window, chunk, keep_first, float(scale),
             float(softcap), sink_ptr,
         ]
-        kernels = 1
-        if self._in_pairs(step, num_heads, num_kv_heads, window, chunk):
+        kernels, pairs = 1, self._in_pairs(step, num_heads, num_kv_heads, window, chunk)
+        if pairs:
             floats = function("distie_attention_prefill_pairs_scratch_floats")(step.max_kv_len, kv.v.shape[-1], self.sm_count)
             scratch = torch.empty(floats, dtype=torch.float32, device=qkv.device) if floats else None  # parts of long portions
             kernels = 2 if floats else 1
@@ -686,6 +686,8 @@ class DeviceKernels(KernelSet):
             return False
         check(code, "attention_prefill_tcgen05")
         self._ran("attention_prefill_tcgen05", kernels)
+        if pairs:
+            self._ran("attention_prefill_pairs", 0)
         return True
 
     def _in_pairs(self, step, num_heads: int, num_kv_heads: int, window: int, chunk: int) -> bool:

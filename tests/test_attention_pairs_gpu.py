@@ -22,12 +22,22 @@ def ks():
     return make_kernels(torch.bfloat16, "cuda:0")
 
 
+def in_pairs(ks, monkeypatch, *args):
+    """The kernel of pairs, whatever the rule would take: it has to be the one that runs."""
+    from distie_b200.kernels import device
+
+    before = ks.kernel_counts.get("attention_prefill_pairs", 0)
+    with monkeypatch.context() as forced:
+        forced.setattr(device.DeviceKernels, "_in_pairs", lambda *args: True)
+        ks.attention(*args)
+    ks.check_errors()
+    assert ks.kernel_counts["attention_prefill_pairs"] == before + 1
+
+
 def run(ks, monkeypatch, heads, kv_heads, head_dim, value_dim, page, tokens, pasts, window=None, chunk=None, keep_first=0, softcap=0.0,
         sink=False, scale=None, keys=None, missing=None):
-    from distie_b200.kernels import device
     from distie_b200.kernels.interface import KvSlot
 
-    monkeypatch.setattr(device, "pairs_pay", lambda *args: True)
     g = torch.Generator(device="cuda").manual_seed(heads * 31 + head_dim + sum(tokens))
     kv = filled_cache_for(torch.bfloat16, kv_heads, head_dim, page, [p + n for p, n in zip(pasts, tokens)])
     values = torch.randn(*kv.k.shape[:3], value_dim, generator=g, device="cuda").to(torch.bfloat16)
@@ -38,14 +48,11 @@ def run(ks, monkeypatch, heads, kv_heads, head_dim, value_dim, page, tokens, pas
     q = torch.randn(step.num_tokens, heads * head_dim, generator=g, device="cuda").to(torch.bfloat16)
     sinks = torch.randn(heads, generator=g, device="cuda") if sink else None
     out = torch.full((step.num_tokens, heads * value_dim), float("nan"), dtype=torch.bfloat16, device="cuda")
-    before = ks.kernel_counts.get("attention_prefill_tcgen05", 0)
     args = (heads, kv_heads, head_dim, window, scale or head_dim**-0.5, chunk, keep_first, softcap, sinks)
     want = ref.attention(q, step, kv, *args)
     if missing is not None:
         missing(kv)
-    ks.attention(q, out, step, kv, *args)
-    ks.check_errors()
-    assert ks.kernel_counts["attention_prefill_tcgen05"] == before + 1
+    in_pairs(ks, monkeypatch, q, out, step, kv, *args)
     close(out, want, torch.bfloat16, f"{heads} heads, {tokens} behind {pasts}")
 
 
@@ -104,9 +111,6 @@ def test_weights_above_the_maximum_in_use_count_as_they_are_rounded(ks, monkeypa
     own rounding (2^-9 at most, 1.1e-3 in the root mean square, of each of 128 elements whose squares weigh as normal numbers' do:
     1.1e-3 (3 / 128)^1/2 = 1.7e-4) and what the other keys' share of 1500 / 2^19 leaves; with weights summed before they are
     rounded, by up to 2^-9 at once."""
-    from distie_b200.kernels import device
-
-    monkeypatch.setattr(device.DeviceKernels, "_in_pairs", lambda *args: True)
     g = torch.Generator(device="cuda").manual_seed(past)
     heads, tokens, at, scale = 4, 200, 32, 128**-0.5  # (keys 512 to 527)
     kv = filled_cache_for(torch.bfloat16, 2, 128, 16, [past + tokens])
@@ -117,8 +121,7 @@ def test_weights_above_the_maximum_in_use_count_as_they_are_rounded(ks, monkeypa
     q[..., 0] = torch.empty(tokens, heads, device="cuda").uniform_(low, high, generator=g) * 0.6931 / (16 * scale)
     q = q.to(torch.bfloat16)
     out = torch.empty(tokens, heads * 128, dtype=torch.bfloat16, device="cuda")
-    ks.attention(q.reshape(tokens, -1), out, step, kv, heads, 2, 128, None, scale)
-    ks.check_errors()
+    in_pairs(ks, monkeypatch, q.reshape(tokens, -1), out, step, kv, heads, 2, 128, None, scale)
     keys = torch.arange(past + tokens, device="cuda")
     pages = kv.block_table[0, keys // 16].long()
     k, v = (c[pages, :, keys % 16].double().repeat_interleave(heads // 2, dim=1) for c in (kv.k, kv.v))
@@ -129,15 +132,29 @@ def test_weights_above_the_maximum_in_use_count_as_they_are_rounded(ks, monkeypa
     assert float(along.square().mean().sqrt()) < 3e-4
 
 
-def test_a_missing_page_sets_the_error_word(ks, monkeypatch):
-    from distie_b200.kernels import device
+@pytest.mark.parametrize("past,missing", [(1300, 40), (1300, 93), (300, 0)])  # in parts of cut units, in a whole one
+def test_a_missing_page_sets_the_error_word(ks, monkeypatch, past, missing):
     from distie_b200.kernels.library import KernelError
 
-    monkeypatch.setattr(device, "pairs_pay", lambda *args: True)
-    kv = filled_cache_for(torch.bfloat16, 2, 128, 16, [1500])
-    kv.block_table[0, 40] = -1
-    step = step_of([200], [1300], [0])
+    kv = filled_cache_for(torch.bfloat16, 2, 128, 16, [past + 200])
+    step = step_of([200], [past], [0])
     q = torch.randn(200, 4 * 128, device="cuda").to(torch.bfloat16)
-    ks.attention(q, torch.empty_like(q), step, kv, 4, 2, 128, None, 128**-0.5)
-    with pytest.raises(KernelError):
+    page, kv.block_table[0, missing] = int(kv.block_table[0, missing]), -1
+    with pytest.raises(KernelError, match="portion of a prompt"):
+        in_pairs(ks, monkeypatch, q, torch.empty_like(q), step, kv, 4, 2, 128, None, 128**-0.5)
+    kv.block_table[0, missing] = page  # and the next call is as if nothing had been
+    out = torch.full_like(q, float("nan"))
+    in_pairs(ks, monkeypatch, q, out, step, kv, 4, 2, 128, None, 128**-0.5)
+    close(out, ref.attention(q, step, kv, 4, 2, 128, None, 128**-0.5), torch.bfloat16, "after a missing page")
+
+
+def test_steps_that_the_rule_sends_to_either_kernel_count_apart(ks):
+    kv = filled_cache_for(torch.bfloat16, 2, 128, 16, [4130])
+    for tokens, past, pairs in ((130, 0, 0), (130, 4000, 1)):
+        step = step_of([tokens], [past], [0])
+        q = torch.randn(tokens, 12 * 128, device="cuda").to(torch.bfloat16)
+        before = [ks.kernel_counts.get(name, 0) for name in ("attention_prefill_tcgen05", "attention_prefill_pairs")]
+        ks.attention(q, torch.empty_like(q), step, kv, 12, 2, 128, None, 128**-0.5)
         ks.check_errors()
+        after = [ks.kernel_counts.get(name, 0) for name in ("attention_prefill_tcgen05", "attention_prefill_pairs")]
+        assert [b - a for a, b in zip(before, after)] == [1, pairs]

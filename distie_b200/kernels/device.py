@@ -124,7 +124,7 @@ def wide_pays(m: int, n: int, k: int, sms: int) -> bool:
     if 6 * (m + n) * k > _CHUNK_BYTES:
         return False
     waves = -(-(-(-m // 128) * -(-n // 128)) // sms)
-    return 6.6 + 2.04e-6 * (m + n) * k + 0.0194 * waves * k < 0.95 * (6.0 + m * n * k * 4e-8)
+    return 7.4 + 2.04e-6 * (m + n) * k + 0.0194 * waves * k < 0.95 * (6.0 + m * n * k * 4e-8)
 
 
 def pairs_pay(portions: list, heads: int, kv_heads: int, window: int, longest: int, sms: int) -> bool:

@@ -71,3 +71,55 @@ def test_numbers_that_are_not_finite_and_the_largest(ks):
     error = (got.double() - x.double() @ w.double().t()).abs() / (x.double().norm(dim=1)[:, None] * w.double().norm(dim=1))
     assert float(error[keep].max()) < 2e-6
     assert float(got[40, 50]) == 3.4028234663852886e38
+
+
+@pytest.mark.parametrize("k", [96, 768, 776, 1544, 6152])  # one, two and eight warps a row, rows read twice
+def test_rows_of_the_smallest_and_largest_numbers_keep_their_bits(ks, k):
+    """Every float32 number has three planes, whatever its size: rows and columns of 2^-149 to 2^127 against 64 bits, as near
+    to them as ordinary ones are (their own last bits are what a row below 2^-126 holds of them)."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    sizes = torch.tensor([-149, -140, -126, -120, -116, -112, -100, -64, -41, -40, -39, 0, 30, 39, 40, 41, 64, 100, 126], device="cuda")
+    x = torch.rand(3 * sizes.numel(), k, generator=g, device="cuda") * 2 - 1
+    w = torch.rand(4 * sizes.numel(), k, generator=g, device="cuda") * 2 - 1
+    x = torch.ldexp(x, sizes.repeat(3)[:, None])
+    w = torch.ldexp(w, sizes.repeat_interleave(4)[:, None])
+    x[:, 5] = torch.where(x.abs().amax(1) == 0, 2.0**-149, x[:, 5])
+    want = x.double() @ w.double().t()
+    got = product(ks, x, w).double()
+    scale = x.double().norm(dim=1)[:, None] * w.double().norm(dim=1)
+    inside = (want.abs() < 3.4e38) & (scale > 0)
+    bound = (8 + (k / 128) ** 0.5) * 2.0**-24 * scale + 2.0**-149
+    assert bool(((got - want).abs() <= bound)[inside].all()), float(((got - want).abs() / bound)[inside].max())
+    beyond = want.abs() > 3.5e38
+    assert torch.equal(got[beyond], want[beyond].sign() * float("inf"))
+
+
+def test_infinity_times_the_smallest_numbers_is_infinity(ks):
+    x, w = torch.ones(200, 64, device="cuda"), torch.ones(128, 64, device="cuda")
+    x[3, 9], w[4, 9], w[5, 9], w[6, 9] = float("inf"), 2.0**-149, -(2.0**-140), 0.0
+    w[7] *= 2.0**127
+    w[7, 9] = -(2.0**-149)
+    got = product(ks, x, w)
+    assert got[3, 4] == float("inf") and got[3, 5] == float("-inf") and bool(got[3, 6].isnan()) and got[3, 7] == float("-inf")
+    assert bool(torch.isfinite(got[:3, :7]).all()) and bool(torch.isfinite(got[4:, :7]).all())
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), 3e38])
+def test_rows_that_are_not_finite_take_no_longer(ks, value):
+    x, w = torch.randn(777, 1536, device="cuda"), torch.randn(2048, 1536, device="cuda")
+    odd = x.clone()
+    odd[::7, 100] = value
+
+    def time(x):
+        best = 1e9
+        for _ in range(10):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            product(ks, x, w)
+            end.record()
+            torch.cuda.synchronize()
+            best = min(best, start.elapsed_time(end))
+        return best
+
+    time(x)
+    assert time(odd) < 2 * time(x)

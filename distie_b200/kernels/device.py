@@ -104,13 +104,20 @@ def grouped_tile(pairs: int, experts: int) -> int:
     """Rows of a tile of the routed products: 128, a CTA each, or 256, a pair of CTAs each, which pulls a third less out of L2
     for the same rows but leaves more of them empty where an expert's rows do not fill a tile.
 
-    1.115: what a row costs more in tiles of 128; the mean and 12 % around it stand for the experts' shares.  Both products of 16
-    experts of 1,536 x 2,240 and all around them, us, in tiles of 128 / 256, at 75, 112, 188, 375, 562 rows an expert on average:
-    89 / 103, 106 / 105, 120 / 110, 174 / 166, 237 / 241; of 3,584 x 4,736: 305 / 390, 337 / 384, 422 / 397, 738 / 674, 1,072 /
-    1,100; a layer with 131 rows an expert 214 / 242."""
-    shares = [share * pairs / experts for share in (0.88, 1.0, 1.12)]
+    Five points of a spread of sqrt(rows), what equal chances give, stand for the experts' shares; 1.185: what a row costs more in
+    tiles of 128.  Of up to eight experts either tile is bound by the weights, which the pairs stream faster.  Fitted to 672
+    layers timed both ways (8, 16 and 64 experts of 1,536 x 2,240, 3,584 x 4,736, 2,048 x 768 and 5,120 x 1,536, 40 to 800 rows an
+    expert, equal chances and uneven ones; hidden and expert sizes moved the ratio less than the rows did): on average 1.5 %
+    over the faster tile, 128 of them more than 3 %, 32 % at most (64 experts of uneven shares; either tile
+    throughout is 3.1 and 3.4 % over).  Layers of 16 experts, us, in tiles of 128 / 256, at 75, 112, 188, 275, 300, 350, 375, 562
+    rows an expert: of 1,536 x 2,240 104 / 115, 119 / 111, 131 / 119, 145 / 162, 166 / 164, 180 / 168, 182 / 168, 244 / 242; of
+    3,584 x 4,736 320 / 389, 373 / 389, 418 / 389, 565 / 676, 662 / 708, 674 / 698, 723 / 709, 1,042 / 1,114."""
+    mean = pairs / experts
+    if experts <= 8 and mean >= 72:
+        return 256
+    shares = [mean + off * math.sqrt(mean) for off in (-1.4, -0.7, 0.0, 0.7, 1.4)]
     by_tile = [sum(math.ceil(rows / tile) * tile for rows in shares) for tile in (128, 256)]
-    return 256 if by_tile[1] < 1.115 * by_tile[0] else 128
+    return 256 if by_tile[1] < 1.185 * by_tile[0] else 128
 
 
 def wide_pays(m: int, n: int, k: int, sms: int) -> bool:

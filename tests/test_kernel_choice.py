@@ -81,6 +81,17 @@ def test_routed_products_take_the_tile_that_is_not_slower(rows, tile):
     assert grouped_tile(16 * rows, 16) == tile
 
 
+@pytest.mark.parametrize("experts,rows,single,pair", [  # us of a layer in tiles of 128 and of 256
+    (8, 112, 76, 72), (8, 131, 76, 74), (8, 150, 84, 74), (8, 275, 106, 102), (8, 375, 111, 104), (8, 420, 119, 106),
+    (16, 40, 313, 352), (16, 75, 320, 389), (16, 169, 422, 406), (16, 220, 428, 403), (16, 275, 565, 676), (16, 300, 662, 708), (16, 330, 678, 715),
+    (16, 375, 182, 168), (16, 375, 723, 709), (16, 420, 862, 776), (16, 562, 1042, 1114), (16, 700, 1231, 1176),
+    (64, 64, 298, 317), (64, 112, 344, 360), (64, 188, 436, 416), (64, 275, 596, 641), (64, 330, 668, 725), (64, 350, 686, 727), (64, 450, 883, 809),
+    (64, 562, 1096, 1114), (64, 700, 1292, 1243),
+])
+def test_routed_products_take_the_tile_that_was_faster(experts, rows, single, pair):
+    assert grouped_tile(experts * rows, experts) == (128 if single < pair else 256)
+
+
 def test_float32_products_that_the_library_refuses_or_spreads_stay_with_it(monkeypatch):
     """Operands that do not fit one another never reach the kernel, which takes its sizes from the weight alone."""
     entered = []

@@ -178,6 +178,7 @@ class DeviceKernels(KernelSet):
             torch.backends.cudnn.allow_tf32 = False
             torch.set_float32_matmul_precision("highest")
         library.load_unit("base")
+        library.load_unit("float32")  # (a bfloat16 engine's too: matrices that a checkpoint stores in 32 bits)
         if dtype == torch.bfloat16:
             library.load_unit("bf16")
         self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count

@@ -123,3 +123,14 @@ def test_rows_that_are_not_finite_take_no_longer(ks, value):
 
     time(x)
     assert time(odd) < 2 * time(x)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_the_kernel_is_loaded_with_the_kernel_set(monkeypatch, dtype):
+    """Not by the first large product, which would wait for the compiler where the unit was not built ahead."""
+    from distie_b200.kernels import library, make_kernels
+
+    seen, load = [], library.load_unit
+    monkeypatch.setattr(library, "load_unit", lambda unit: seen.append(unit) or load(unit))
+    make_kernels(dtype, "cuda:0")
+    assert "float32" in seen

@@ -195,6 +195,13 @@ class DeviceKernels(KernelSet):
         self.launches += kernels
         self.kernel_counts[name] = self.kernel_counts.get(name, 0) + 1
 
+    def _scratch(self, floats: int) -> torch.Tensor | None:
+        """Scratch of a kernel that another one can stand in for; None where the memory that is left does not hold it."""
+        try:
+            return torch.empty(floats, dtype=torch.float32, device=self.error_flag.device)
+        except torch.OutOfMemoryError:
+            return None
+
     def check_errors(self) -> None:
         code = int(self.error_flag.item())
         if code:
@@ -310,8 +317,10 @@ class DeviceKernels(KernelSet):
             return None
         if any(t.device != self.error_flag.device or (t.requires_grad and torch.is_grad_enabled()) for t in operands):
             return None
+        scratch = self._scratch(function("distie_gemm_float32_scratch_floats")(m, n, k))
+        if scratch is None:
+            return None
         out = torch.empty((m, n), dtype=torch.float32, device=x.device)
-        scratch = torch.empty(function("distie_gemm_float32_scratch_floats")(m, n, k), dtype=torch.float32, device=x.device)
         code = function("distie_gemm_float32")(
             x.data_ptr(), x.stride(0), weight.data_ptr(), bias.data_ptr() if bias is not None else None, out.data_ptr(), n, m, n, k,
             scratch.data_ptr(), self.error_flag.data_ptr(), self._stream(),
@@ -681,11 +690,13 @@ class DeviceKernels(KernelSet):
             num_heads, num_kv_heads, head_dim, kv.v.shape[-1], kv.page_size, kv.num_pages, window, chunk, keep_first, float(scale),
             float(softcap), sink_ptr,
         ]
-        kernels, pairs = 1, self._in_pairs(step, num_heads, num_kv_heads, window, chunk)
+        kernels, scratch, pairs = 1, None, self._in_pairs(step, num_heads, num_kv_heads, window, chunk)
+        floats = function("distie_attention_prefill_pairs_scratch_floats")(step.max_kv_len, kv.v.shape[-1], self.sm_count) if pairs else 0
+        if floats:  # parts of long portions
+            kernels, scratch = 2, self._scratch(floats)
+        if pairs and floats and scratch is None:
+            kernels, pairs = 1, False
         if pairs:
-            floats = function("distie_attention_prefill_pairs_scratch_floats")(step.max_kv_len, kv.v.shape[-1], self.sm_count)
-            scratch = torch.empty(floats, dtype=torch.float32, device=qkv.device) if floats else None  # parts of long portions
-            kernels = 2 if floats else 1
             code = function("distie_attention_prefill_pairs")(*args, scratch.data_ptr() if floats else None, self.sm_count,
                                                               self.error_flag.data_ptr(), self._stream())
         else:

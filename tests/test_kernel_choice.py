@@ -92,14 +92,21 @@ def test_routed_products_take_the_tile_that_was_faster(experts, rows, single, pa
     assert grouped_tile(experts * rows, experts) == (128 if single < pair else 256)
 
 
-def test_float32_products_that_the_library_refuses_or_spreads_stay_with_it(monkeypatch):
-    """Operands that do not fit one another never reach the kernel, which takes its sizes from the weight alone."""
+@pytest.fixture
+def fake(monkeypatch):
+    """A float32 kernel set on the CPU whose entries are only noted down; every float32 product pays."""
     entered = []
     monkeypatch.setattr(device, "wide_pays", lambda *args: True)
     monkeypatch.setattr(device, "function", lambda name: lambda *args: entered.append(name) or 0)
     ks = device.DeviceKernels.__new__(device.DeviceKernels)
     ks.dtype, ks.sm_count, ks.error_flag, ks.launches, ks.kernel_counts = torch.float32, 148, torch.zeros(1, dtype=torch.int32), 0, {}
     ks._stream = lambda: 0
+    return ks, entered
+
+
+def test_float32_products_that_the_library_refuses_or_spreads_stay_with_it(fake):
+    """Operands that do not fit one another never reach the kernel, which takes its sizes from the weight alone."""
+    ks, entered = fake
     x, w = torch.ones(200, 64), torch.ones(128, 64)
     ks.linear(x, w, torch.ones(128))
     assert entered and ks.kernel_counts == {"gemm_float32": 1}
@@ -117,3 +124,30 @@ def test_float32_products_that_the_library_refuses_or_spreads_stay_with_it(monke
     grown = torch.ones(128, 64, requires_grad=True)
     ks.linear(x, grown).sum().backward()
     assert torch.equal(grown.grad, torch.full((128, 64), 200.0)) and not entered
+
+
+def test_scratch_that_the_memory_does_not_hold_leaves_the_work_to_the_other_kernel(fake, monkeypatch):
+    from distie_b200.kernels.interface import KvSlot, StepTensors
+
+    ks, entered = fake
+    sizes = {"distie_gemm_float32_scratch_floats": 1 << 50, "distie_attention_prefill_pairs_scratch_floats": 1 << 50}
+    monkeypatch.setattr(device, "function", lambda name: lambda *args: entered.append(name) or sizes.get(name, 0))
+
+    def full(*size, **kw):
+        if size[0] == 1 << 50:
+            raise torch.OutOfMemoryError("full")
+        return torch.zeros(*size, **kw)
+
+    monkeypatch.setattr(device.torch, "empty", full)
+    assert torch.equal(ks.linear(torch.ones(200, 64), torch.ones(128, 64)), torch.full((200, 128), 64.0))
+    assert entered == ["distie_gemm_float32_scratch_floats"]
+    entered.clear()
+    monkeypatch.setattr(device.DeviceKernels, "_in_pairs", lambda *args: True)
+    ids = torch.zeros(2, dtype=torch.int32)
+    step = StepTensors(token_ids=ids, positions=ids, token_seq=ids, seq_seat=ids, num_tokens=2, num_seqs=1, num_decode_tokens=0, max_kv_len=2)
+    step.q_tiles, step.num_q_tiles = torch.tensor([[0, 2]], dtype=torch.int32), 1
+    cache = torch.zeros(1, 1, 16, 64)
+    q = torch.zeros(2, 64)
+    assert ks._attention_tcgen05(q, q, step, KvSlot(cache, cache, ids[None], 16, 1), 1, 1, 64, 0, 0, 0.125)
+    assert entered == ["distie_attention_prefill_pairs_scratch_floats", "distie_attention_prefill_tcgen05"]
+    assert ks.kernel_counts == {"attention_prefill_tcgen05": 1} and ks.launches == 1

@@ -106,7 +106,10 @@ struct PairPiece {
   int halves;      // tiles of it: 2, or 1 where no second one goes with the first
   int slot;        // of the scratch that takes it; -1: the whole unit
   int stop;        // no piece: the CTA's work is done
-  int pad;
+  // Blocks that hold keys for a tile, where two tiles share the unit: the first one sees those before `seen_end`, the second one
+  // all but [gap_from, gap_to), between the kept keys and its window.  Products with the others are left out: 0 * (what is
+  // not finite) is not 0.
+  int seen_end, gap_from, gap_to;
 };
 
 template <int DK, int DV>
@@ -490,6 +493,14 @@ attention_prefill_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const 
           if (some || last) break;
         }
         const PairWalk walk(p.stop ? 0 : p.pos0[0], p.stop ? 0 : p.pos0[1] + p.rows[1] - 1, a.window, a.key_chunk, a.keep_first);
+        p.seen_end = 0x7fffffff;
+        p.gap_from = p.gap_to = 0;
+        if (!p.stop && g.tiles == 2) {
+          const int at_first = walk.sink_blocks - walk.block_first;  // from a block of keys to its place in the walk
+          p.seen_end = at_first + (g.pos0 + g.rows - 1) / kPairKeys + 1;
+          p.gap_from = at_first + max(walk.block_first, (a.keep_first + kPairKeys - 1) / kPairKeys);
+          p.gap_to = at_first + first_visible_key(g.pos0 + g.rows, a.window, a.key_chunk) / kPairKeys;
+        }
         bool mine = false;
         const int page = p.stop ? -1 : page_of(walk, p.seat, p.first, mine);
         if (!waited) {
@@ -566,6 +577,8 @@ attention_prefill_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const 
         const int r = pieces % kPairRing;
         if (!wait_all(&sm.ring_full[r], (pieces / kPairRing) & 1)) { ok = false; break; }
         const int n = sm.ring[r].end - sm.ring[r].first, halves = sm.ring[r].halves, stop = sm.ring[r].stop;
+        const int seen_end = sm.ring[r].seen_end - sm.ring[r].first, gap_from = sm.ring[r].gap_from - sm.ring[r].first;
+        const int gap_to = sm.ring[r].gap_to - sm.ring[r].first, first1 = gap_from <= 0 ? max(0, gap_to) : 0;  // (the second tile's first)
         // Where the output tile goes through the place of Q, the store hands that back.
         const bool plain = sm.ring[r].slot >= 0 || a.value_dim != DV;
         const bool frees_q[2] = {plain || sm.ring[r].rows[0] != kPairRows, plain || sm.ring[r].rows[1] != kPairRows};
@@ -586,14 +599,18 @@ attention_prefill_pairs_kernel(const __grid_constant__ CUtensorMap map_q, const 
             const uint32_t s_cols = tmem + h * kPairKeys, o_cols = tmem + O_COL + h * DV;
             const uint32_t phase = (h == 0 ? cnt[0] : cnt[1]) & 1;
             if (j >= 0) {  // O of the tile += P V of block j of the piece
+              const bool sees = h == 0 ? j < seen_end : j < gap_from || j >= gap_to;
+              const uint32_t add = j > (h == 0 ? 0 : first1) ? 1u : 0u;
 #pragma unroll
               for (int part = 0; part < 2; ++part) {
                 if (!wait_all(&sm.p_full[h][part], phase)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (elect_one()) {
+                  if (sees) {
 #pragma unroll
-                  for (int kk = part * 4; kk < part * 4 + 4; ++kk)  // 16 keys: 8 columns of P, 16 rows of V
-                    umma_bf16_ts(o_cols, s_cols + kk * 8, v_desc + (uint64_t)((kk * 16 * 128) >> 4), idesc_o, kk > 0 ? 1u : (j > 0 ? 1u : 0u));
+                    for (int kk = part * 4; kk < part * 4 + 4; ++kk)  // 16 keys: 8 columns of P, 16 rows of V
+                      umma_bf16_ts(o_cols, s_cols + kk * 8, v_desc + (uint64_t)((kk * 16 * 128) >> 4), idesc_o, kk > 0 ? 1u : add);
+                  }
                   umma_commit(&sm.pv_done[h][part]);
                   if (part == 1 && h == halves - 1) umma_commit(&sm.v_empty[vs]);
                 }
@@ -909,7 +926,8 @@ __global__ void __launch_bounds__(256) merge_pairs_kernel(const __grid_constant_
 #pragma unroll
     for (int c = 0; c < OWN; ++c) v[c] = __ldcg(reinterpret_cast<const float4*>(part) + (warp * OWN + c) * kPairRows + row);
     const float m = __ldcg(part + kPairRows * DV + row);
-    const float w = m == -INFINITY ? 0.f : exp2_approx(m - top);
+    if (m == -INFINITY) continue;  // (a part without a key for this row: where its tile sees none at all, O was not written)
+    const float w = exp2_approx(m - top);
     sum += w * __ldcg(part + kPairRows * (DV + 1) + row);
 #pragma unroll
     for (int c = 0; c < OWN; ++c) {

@@ -132,6 +132,31 @@ def test_weights_above_the_maximum_in_use_count_as_they_are_rounded(ks, monkeypa
     assert float(along.square().mean().sqrt()) < 3e-4
 
 
+@pytest.mark.parametrize("past,tokens,window,keep_first,at,free", [
+    (0, 200, None, 0, 190, slice(0, 128)), (70, 300, None, 0, 330, slice(0, 128)), (70, 300, None, 0, 260, slice(0, 128)),
+    (4990, 200, None, 0, 5150, slice(0, 128)),  # (cut: a piece may end with blocks that the first tile does not see)
+    (100, 256, 100, 0, 50, slice(128, 256)), (100, 256, None, 0, 50, slice(0, 0)), (3000, 256, 100, 0, 2930, slice(128, 256)),
+    (3000, 256, 100, 200, 2930, slice(128, 256)), (100, 256, 30, 40, 100, slice(0, 0)), (300, 256, 100, 129, 230, slice(0, 0)),
+    (600, 256, 300, 400, 390, slice(0, 0)), (650, 256, 100, 300, 560, slice(128, 256)),
+])
+@pytest.mark.parametrize("heads", [1, 7])
+def test_a_value_that_is_not_finite_stays_with_the_tiles_that_see_its_block(ks, monkeypatch, heads, past, tokens, window, keep_first, at, free):
+    """Two tiles of one request share a unit; blocks of keys that only one of them sees leave the other one's rows alone."""
+    kv = filled_cache_for(torch.bfloat16, 1, 128, 16, [past + tokens])
+    step = step_of([tokens], [past], [0])
+    q = torch.randn(tokens, heads * 128, device="cuda").to(torch.bfloat16)
+    args = (heads, 1, 128, window, 128**-0.5, None, keep_first)
+    want = ref.attention(q, step, kv, *args)
+    kv.v[int(kv.block_table[0, at // 16]), :, at % 16] = float("nan")
+    out = torch.zeros_like(q)
+    in_pairs(ks, monkeypatch, q, out, step, kv, *args)
+    if out[free].numel():
+        close(out[free], want[free], torch.bfloat16)
+    sees = torch.arange(past, past + tokens, device="cuda")
+    sees = (sees >= at) & ((sees - at < (window or 1 << 30)) | (at < keep_first))
+    assert bool(out[sees].isnan().all())
+
+
 @pytest.mark.parametrize("past,missing", [(1300, 40), (1300, 93), (300, 0)])  # in parts of cut units, in a whole one
 def test_a_missing_page_sets_the_error_word(ks, monkeypatch, past, missing):
     from distie_b200.kernels.library import KernelError

@@ -18,12 +18,12 @@
 //   MMA order        PV0(j), S0(j + 1), PV1(j), S1(j + 1): the S that overwrites a block's P is issued behind the products
 //                    that read it (MMAs of one thread execute in the order of issue)
 //
-// Measured (28 heads of 128 in groups of 7, 1,733 tokens of three requests behind 7,000): 222 us against 391 with a tile a CTA,
-// 0.85 PFLOP/s.  A block of both tiles takes 3,430 cycles, and either tile's chain is what they are: 1,000 for each half of the
+// Measured (28 heads of 128 in groups of 7, 1,733 tokens of three requests behind 7,000): 231 us against 373 with a tile a CTA,
+// 0.79 PFLOP/s.  A block of both tiles takes 3,600 cycles, and either tile's chain is what they are: 1,100 for each half of the
 // exponentials (512 of the special-function unit; the scores, the sums and the way back into tensor memory are the rest), 250
-// to wake the issuer, 900 for the products.  Sixteen softmax warps with half of a row each (4,150 cycles), a search for the
-// maximum in every block (3,800), a rolled loop over the halves (4,300: copies of the scores) and polling without sleep (3,600)
-// were slower.
+// to wake the issuer, 900 for the products.  Measured while the sums were of unrounded weights, 3,430 cycles a block:
+// sixteen softmax warps with half of a row each 4,150, a search for the maximum in every block 3,800, a rolled loop over the
+// halves 4,300 (copies of the scores), polling without sleep 3,600.
 //
 // Work is shared out among at most one CTA an SM by key blocks, not by tiles.  Every CTA reads the step's tiles and finds its
 // part itself (a warp, before the wait for the kernel ahead):

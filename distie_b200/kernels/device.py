@@ -142,8 +142,9 @@ def pairs_pay(portions: list, heads: int, kv_heads: int, window: int, longest: i
     48 heads in groups of 1 to 8, heads of 64 and 128, 1 to 32 portions of 2 to 3,000 tokens behind up to 9,000, windows).  A
     tile to itself takes a block in less time than one of a pair does, so steps whose longest tile takes the time are the
     first kernel's, and steps with work for all SMs, or with long rows of keys that can be cut, the second one's (us, one /
-    two tiles a CTA: 12 heads, 2,048 tokens 30.7 / 33.5; 28 heads, 2,048 behind 4,000 253 / 150; 12 heads, 130 behind 6,000 76 / 33;
-    28 heads, 64 portions of 2 behind 100 99 / 49; 64 tokens behind 200 12 / 17).  0.9: where the estimates err."""
+    two tiles a CTA: 12 heads, 2,048 tokens 31 / 36; 28 heads, 2,048 behind 4,000 253 / 160; 12 heads, 130 behind 6,000 77 / 36;
+    28 heads, 64 portions of 2 behind 100 100 / 51; 64 tokens behind 200 13 / 18).  0.9: where the estimates err; 700 other steps
+    timed since the kernel of pairs sums rounded weights (5 % slower): 4 sent to the slower kernel by more than 3 %, 11 % at most."""
     tiles = blocks = most = 0
     for past, tokens in portions:
         count, first = -(-tokens // 128), (past + 127) // 128 + 1  # tiles, and the blocks that the first of them sees

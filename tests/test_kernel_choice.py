@@ -54,15 +54,15 @@ def test_float32_attention_runs_in_tiles_where_that_is_faster(heads, size, porti
 
 @pytest.mark.parametrize("heads,kv_heads,window,portions,one,two", [
     # heads, those of keys, window, (cached, new) tokens of the portions, us with one and with two tiles a CTA
-    (12, 2, 0, [(0, 130)], 10.3, 12.5),
-    (12, 2, 0, [(6000, 130)], 76.3, 33.0),
-    (12, 2, 0, [(0, 1024)], 18.4, 22.9),
-    (12, 2, 0, [(9000, 1000)], 123.1, 72.2),
-    (28, 4, 0, [(4000, 2048)], 252.9, 149.8),
-    (28, 4, 0, [(100, 2)] * 64, 99.2, 48.6),
-    (40, 8, 0, [(200, 64)], 12.6, 17.4),
-    (7, 1, 0, [(0, 777)], 17.2, 21.5),
-    (8, 8, 0, [(0, 128)] * 16, 7.8, 10.8),
+    (12, 2, 0, [(0, 130)], 10.9, 13.4),
+    (12, 2, 0, [(6000, 130)], 76.9, 36.3),
+    (12, 2, 0, [(0, 1024)], 18.8, 24.9),
+    (12, 2, 0, [(9000, 1000)], 123.1, 77.3),
+    (28, 4, 0, [(4000, 2048)], 253.3, 160.2),
+    (28, 4, 0, [(100, 2)] * 64, 99.6, 50.7),
+    (40, 8, 0, [(200, 64)], 13.1, 17.7),
+    (7, 1, 0, [(0, 777)], 17.5, 23.2),
+    (8, 8, 0, [(0, 128)] * 16, 9.2, 12.8),
 ])
 def test_prompt_attention_takes_two_tiles_a_cta_where_that_is_faster(heads, kv_heads, window, portions, one, two):
     assert pairs_pay(portions, heads, kv_heads, window, max(p + n for p, n in portions), 148) == (two < one)
